@@ -1,16 +1,26 @@
 // Decode-step attention against a padded key/value cache: one query token per sequence, all query heads of a
-// key/value head handled by one CTA so every cached key and value is read from HBM exactly once.
+// key/value head handled together so every cached key and value is read from HBM exactly once.
 //
 //   cache layout  k, v: [batch, max_len, kv_heads, head_dim] bf16 (one layer's slice)
 //   q:                  [batch, heads * head_dim] bf16        cols[b]: index of the newest key of sequence b
 //   out[b, h, :] = softmax_j<=cols[b](scale * <q[b, h], k[b, j, h / G]>) @ v[b, j, h / G]
 //
-// grid (batch, kv_heads), 4 warps. A warp owns keys j = warp, warp + 4, ...; its lanes split head_dim, so a key row
-// is one coalesced 128- or 256-byte read, the G dot products are lane-partial sums folded by shuffles, and every
-// warp keeps an online-softmax state (max, sum, accumulator) per query head in registers. The four states are merged
-// through shared memory at the end. The step is memory-bound: the cache is streamed once, nothing is written but
-// the output row. Sequence lengths are read on the device - the host never synchronises on them.
+// What bounds it: the cache is streamed once, nothing is written but the output row, so HBM bandwidth is the floor. Three
+// things decide how close a kernel comes. (1) Enough blocks: a (sequence, key/value head) pair is cut over a CLUSTER of
+// blocks, each of which takes an equal, 16-key aligned part of that sequence's keys; the parts' softmax states are merged
+// through distributed shared memory, so there is no workspace and no second launch. (2) Bytes in flight: every warp runs
+// its own cp.async ring of 16-key tiles and never meets a block barrier inside the loop. (3) Arithmetic off the critical
+// path: the group's G query heads against 16 keys are a 16 x 16 x head_dim product, done with mma.sync (a memory-bound
+// kernel needs 2 % of the tensor rate; tcgen05's 128-row tiles would be mostly padding).
 //
+// Precision: queries, keys and values are bf16 already, sums and softmax are fp32. The probabilities stay fp32 in effect:
+// each is split into two bf16 terms (p = hi + lo to 2^-17) that go through the same product. With G <= 8 the split is
+// free: the product has 16 rows, the heads use rows 0-7 and the low terms ride in rows 8-15.
+//
+// Measured (B200, 64 sequences of 2,000-8,000 keys, 32 / 4 heads of 128: 655 MB of cache): 3,662 us before (one block of
+// four warps per pair, shuffles and scalar products), 106 us now = 6.1 TB/s of cache (0.93 of the measured copy rate).
+//
+// Sequence lengths are read on the device - the host never synchronises on them.
 // Stands where the reference's rollout engines run their paged decode kernels; here the cache is the sampler's own
 // (halo_b200/inference/generate.py).
 #include "sm100_common.cuh"
@@ -22,110 +32,329 @@ namespace decode {
 
 constexpr int kWarps = 4;
 constexpr int kMaxGroup = 16;      // query heads per key/value head
+constexpr int kTileKeys = 16;      // keys per warp and step
+constexpr int kStages = 3;         // ring depth per warp: 2 blocks of 96 KB per SM keep 128 KB of loads in flight
 
-template <int DPL>
-__device__ __forceinline__ void load_row(const __nv_bfloat16* p, float (&f)[DPL]);
-template <>
-__device__ __forceinline__ void load_row<4>(const __nv_bfloat16* p, float (&f)[4]) {
-    const uint2 u = *reinterpret_cast<const uint2*>(p);
-    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.x));
-    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u.y));
-    f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool live) {
+    const int bytes = live ? 16 : 0;    // 0: the 16 bytes are filled with zeros, nothing is read
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
-template <>
-__device__ __forceinline__ void load_row<2>(const __nv_bfloat16* p, float (&f)[2]) {
-    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
-    f[0] = a.x; f[1] = a.y;
+__device__ __forceinline__ void ldmatrix4(uint32_t a, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
+}
+__device__ __forceinline__ void ldmatrix4_trans(uint32_t a, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
+}
+// c += a (16 x 16) * b (16 x 8)
+__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+                 "{%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float ld_cluster(uint32_t local_addr, uint32_t rank) {
+    uint32_t a;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local_addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
 }
 
-// DPL = head_dim / 32 (dims per lane): 4 for head_dim 128, 2 for head_dim 64
-template <int DPL>
-__global__ void __launch_bounds__(kWarps * 32)
+template <int D>
+__host__ __device__ constexpr int ring_bytes() { return kWarps * kStages * kTileKeys * D * 2 * 2; }
+// per-warp partial states, laid over the ring once the loop is over: m, l [kMaxGroup] and acc [kMaxGroup][D] fp32
+template <int D>
+__host__ __device__ constexpr int state_floats() { return 2 * kMaxGroup + kMaxGroup * D; }
+
+// SPLIT2: groups of more than 8 heads use all 16 rows of the product, so the low terms need a product of their own
+template <int D, bool SPLIT2>
+__global__ void __launch_bounds__(kWarps * 32, 2)
 decode_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ kc,
                         const __nv_bfloat16* __restrict__ vc, const long long* __restrict__ cols,
-                        __nv_bfloat16* __restrict__ out, int n_heads, int n_kv_heads, long long max_len, float scale) {
-    constexpr int D = 32 * DPL;
-    __shared__ float s_m[kWarps][kMaxGroup];
-    __shared__ float s_l[kWarps][kMaxGroup];
-    __shared__ float s_acc[kWarps][kMaxGroup][D];
-    const int b = blockIdx.x, hk = blockIdx.y;
+                        __nv_bfloat16* __restrict__ out, int n_heads, int n_kv_heads, long long max_len, float scale,
+                        int parts) {
+    static_assert(kWarps * state_floats<D>() * 4 <= ring_bytes<D>(), "the partial states fit over the ring");
+    extern __shared__ __align__(128) uint8_t smem[];
+    const uint32_t base = smem_u32(smem);
+    constexpr int kRow = D * 2;                     // bytes of a key
+    constexpr int kTile = kTileKeys * kRow;         // bytes of a warp's key (or value) tile
+    constexpr int kChunks = D / 8;                  // 16-byte chunks per row
+    const int b = blockIdx.z, hk = blockIdx.y;
+    const uint32_t part = cluster_rank();
     const int G = n_heads / n_kv_heads;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = lane >> 2, t = lane & 3;          // fragment row and column pair of this lane
     long long n_keys = cols[b] + 1;
-    if (n_keys > max_len) n_keys = max_len;          // never read past the cache, whatever the host passed
+    if (n_keys > max_len) n_keys = max_len;         // never read past the cache, whatever the host passed
     if (n_keys < 1) n_keys = 1;
-    const long long key_stride = (long long)n_kv_heads * D;
-    const __nv_bfloat16* kb = kc + ((long long)b * max_len) * key_stride + (long long)hk * D + lane * DPL;
-    const __nv_bfloat16* vb = vc + ((long long)b * max_len) * key_stride + (long long)hk * D + lane * DPL;
+    // this block's keys: an equal share in whole tiles
+    const long long tiles = (n_keys + kTileKeys - 1) / kTileKeys;
+    const long long share = (tiles + parts - 1) / parts;
+    const long long tile_lo = min(tiles, share * part), tile_hi = min(tiles, tile_lo + share);
+    const int mine = (int)max(0ll, (tile_hi - tile_lo - warp + kWarps - 1) / kWarps);   // tiles tile_lo + warp + 4 i
 
-    float qf[kMaxGroup][DPL], acc[kMaxGroup][DPL], m[kMaxGroup], l[kMaxGroup];
+    const long long key_stride = (long long)n_kv_heads * D;
+    const __nv_bfloat16* kb = kc + (long long)b * max_len * key_stride + (long long)hk * D;
+    const __nv_bfloat16* vb = vc + (long long)b * max_len * key_stride + (long long)hk * D;
+    const uint32_t ring = base + warp * (kStages * 2 * kTile);
+
+    auto load_tile = [&](int i) {
+        if (i < mine) {
+            const long long k0 = (tile_lo + warp + (long long)i * kWarps) * kTileKeys;
+            const uint32_t dst = ring + (i % kStages) * 2 * kTile;
 #pragma unroll
-    for (int g = 0; g < kMaxGroup; ++g) {
-        m[g] = -INFINITY;
-        l[g] = 0.f;
-#pragma unroll
-        for (int d = 0; d < DPL; ++d) {
-            acc[g][d] = 0.f;
-            qf[g][d] = 0.f;
-        }
-        if (g < G) load_row<DPL>(q + ((long long)b * n_heads + (long long)hk * G + g) * D + lane * DPL, qf[g]);
-    }
-    for (long long j = warp; j < n_keys; j += kWarps) {
-        float kf[DPL], vf[DPL];
-        load_row<DPL>(kb + j * key_stride, kf);
-        load_row<DPL>(vb + j * key_stride, vf);
-#pragma unroll
-        for (int g = 0; g < kMaxGroup; ++g) {
-            if (g < G) {
-                float s = 0.f;
-#pragma unroll
-                for (int d = 0; d < DPL; ++d) s += qf[g][d] * kf[d];
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-                s *= scale;
-                const float m_new = fmaxf(m[g], s);
-                const float corr = __expf(m[g] - m_new);       // exp(-inf) = 0 on the first key
-                const float p = __expf(s - m_new);
-                l[g] = l[g] * corr + p;
-#pragma unroll
-                for (int d = 0; d < DPL; ++d) acc[g][d] = acc[g][d] * corr + p * vf[d];
-                m[g] = m_new;
+            for (int c = 0; c < kTileKeys * kChunks / 32; ++c) {
+                const int u = c * 32 + lane, r = u / kChunks, ch = u % kChunks;
+                const bool live = k0 + r < n_keys;
+                const long long off = (live ? k0 + r : 0) * key_stride + ch * 8;
+                const uint32_t d = dst + r * kRow + ((ch ^ (r & 7)) << 4);     // chunks swizzled by row
+                cp_async16(d, kb + off, live);
+                cp_async16(d + kTile, vb + off, live);
             }
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");                   // empty groups keep the count uniform
+    };
+#pragma unroll
+    for (int i = 0; i < kStages - 1; ++i) load_tile(i);
+
+    // query fragments: row g is head g (and g + 8: the head again, so that its low terms find their scores in place)
+    uint32_t qa[D / 16][4];
+    {
+        const __nv_bfloat16* qb = q + ((long long)b * n_heads + (long long)hk * G) * D;
+        const int r0 = g, r1 = SPLIT2 ? g + 8 : g;
+#pragma unroll
+        for (int ks = 0; ks < D / 16; ++ks) {
+            const int c = ks * 16 + t * 2;
+            qa[ks][0] = r0 < G ? *reinterpret_cast<const uint32_t*>(qb + (long long)r0 * D + c) : 0u;
+            qa[ks][1] = r1 < G ? *reinterpret_cast<const uint32_t*>(qb + (long long)r1 * D + c) : 0u;
+            qa[ks][2] = r0 < G ? *reinterpret_cast<const uint32_t*>(qb + (long long)r0 * D + c + 8) : 0u;
+            qa[ks][3] = r1 < G ? *reinterpret_cast<const uint32_t*>(qb + (long long)r1 * D + c + 8) : 0u;
+        }
     }
+    float o[D / 8][4];
 #pragma unroll
-    for (int g = 0; g < kMaxGroup; ++g) {
-        if (g < G) {
-            if (lane == 0) {
-                s_m[warp][g] = m[g];
-                s_l[warp][g] = l[g];
+    for (int n = 0; n < D / 8; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[n][e] = 0.f;
+    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;      // rows g and g + 8
+    const float c_log2 = scale * 1.4426950408889634f;
+
+    for (int i = 0; i < mine; ++i) {
+        load_tile(i + kStages - 1);
+        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 1) : "memory");
+        __syncwarp();
+        const uint32_t sk = ring + (i % kStages) * 2 * kTile, sv = sk + kTile;
+        const long long k0 = (tile_lo + warp + (long long)i * kWarps) * kTileKeys;
+        float s[2][4];                              // scores: keys 0-7 and 8-15 of the tile
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[n][e] = 0.f;
+        {
+            // matrices of one ldmatrix: (keys 0-7, d 0-7), (keys 0-7, d 8-15), (keys 8-15, d 0-7), (keys 8-15, d 8-15)
+            const int r = (lane & 7) + ((lane >> 4) << 3), hi = (lane >> 3) & 1;
+#pragma unroll
+            for (int ks = 0; ks < D / 16; ++ks) {
+                uint32_t kf[4];
+                ldmatrix4(sk + r * kRow + (((2 * ks + hi) ^ (r & 7)) << 4), kf);
+                mma16816(s[0], qa[ks], kf[0], kf[1]);
+                mma16816(s[1], qa[ks], kf[2], kf[3]);
             }
+        }
 #pragma unroll
-            for (int d = 0; d < DPL; ++d) s_acc[warp][g][lane * DPL + d] = acc[g][d];
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[n][e] *= c_log2;      // base-2 logits
+        if (k0 + kTileKeys > n_keys) {
+            const int lim = (int)(n_keys - k0);
+#pragma unroll
+            for (int n = 0; n < 2; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (n * 8 + t * 2 + (e & 1) >= lim) s[n][e] = -INFINITY;
+        }
+        float x0 = fmaxf(fmaxf(s[0][0], s[0][1]), fmaxf(s[1][0], s[1][1]));
+        float x1 = fmaxf(fmaxf(s[0][2], s[0][3]), fmaxf(s[1][2], s[1][3]));
+#pragma unroll
+        for (int sh = 1; sh < 4; sh <<= 1) {
+            x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, sh));
+            x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, sh));
+        }
+        // every tile holds at least one visible key, so the new maxima are finite
+        const float n0 = fmaxf(m0, x0), n1 = fmaxf(m1, x1);
+        if (__any_sync(0xffffffffu, n0 > m0 || n1 > m1)) {
+            const float a0 = exp2f(m0 - n0), a1 = exp2f(m1 - n1);
+            l0 *= a0;
+            l1 *= a1;
+#pragma unroll
+            for (int n = 0; n < D / 8; ++n) {
+                o[n][0] *= a0; o[n][1] *= a0;
+                o[n][2] *= a1; o[n][3] *= a1;
+            }
+            m0 = n0;
+            m1 = n1;
+        }
+        float p[2][4];
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+            p[n][0] = exp2f(s[n][0] - m0); p[n][1] = exp2f(s[n][1] - m0);
+            p[n][2] = exp2f(s[n][2] - m1); p[n][3] = exp2f(s[n][3] - m1);
+        }
+        l0 += (p[0][0] + p[0][1]) + (p[1][0] + p[1][1]);
+        l1 += (p[0][2] + p[0][3]) + (p[1][2] + p[1][3]);
+        // the probabilities as the A operand: hi terms, and what rounding left over as lo terms
+        uint32_t pa[4], pl[4];
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+#pragma unroll
+            for (int hrow = 0; hrow < 2; ++hrow) {
+                const float u = p[n][2 * hrow], v = p[n][2 * hrow + 1];
+                // hi: the upper half of the word (truncated, so that lo >= 0); lo is kept above zero so that an infinite
+                // value stays infinite instead of meeting a zero
+                const uint32_t ub = __float_as_uint(u), vbits = __float_as_uint(v);
+                const uint32_t hi = __byte_perm(ub, vbits, 0x7632);
+                const uint32_t lo = pack_bf16(fmaxf(u - __uint_as_float(ub & 0xFFFF0000u), 1.17549435e-38f),
+                                              fmaxf(v - __uint_as_float(vbits & 0xFFFF0000u), 1.17549435e-38f));
+                if (SPLIT2) {
+                    pa[2 * n + hrow] = hi;
+                    pl[2 * n + hrow] = lo;
+                } else {
+                    pa[2 * n + hrow] = hrow ? lo : hi;     // rows 8-15 repeat the heads: they carry the low terms
+                }
+            }
+        }
+        {
+            // value fragments (transposed load): (keys 0-7, d 0-7), (keys 8-15, d 0-7), (keys 0-7, d 8-15), (keys 8-15, d 8-15)
+            const int r = (lane & 7) + (((lane >> 3) & 1) << 3), hi = lane >> 4;
+#pragma unroll
+            for (int n = 0; n < D / 16; ++n) {
+                uint32_t vf[4];
+                ldmatrix4_trans(sv + r * kRow + (((2 * n + hi) ^ (r & 7)) << 4), vf);
+                mma16816(o[2 * n], pa, vf[0], vf[1]);
+                mma16816(o[2 * n + 1], pa, vf[2], vf[3]);
+                if (SPLIT2) {
+                    mma16816(o[2 * n], pl, vf[0], vf[1]);
+                    mma16816(o[2 * n + 1], pl, vf[2], vf[3]);
+                }
+            }
+        }
+        __syncwarp();                               // every lane is done with the tile before its slot is refilled
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+    for (int sh = 1; sh < 4; sh <<= 1) {
+        l0 += __shfl_xor_sync(0xffffffffu, l0, sh);
+        l1 += __shfl_xor_sync(0xffffffffu, l1, sh);
+    }
+    __syncthreads();                                // the ring is dead: partial states take its place
+    float* st = reinterpret_cast<float*>(smem);
+    {
+        float* w = st + warp * state_floats<D>();
+        if (t == 0) {
+            w[g] = m0;
+            w[kMaxGroup + g] = l0;
+            if (SPLIT2) {
+                w[g + 8] = m1;
+                w[kMaxGroup + g + 8] = l1;
+            }
+        }
+#pragma unroll
+        for (int n = 0; n < D / 8; ++n) {
+            float* row = w + 2 * kMaxGroup + g * D + n * 8 + t * 2;
+            if (SPLIT2) {
+                *reinterpret_cast<float2*>(row) = make_float2(o[n][0], o[n][1]);
+                *reinterpret_cast<float2*>(row + 8 * D) = make_float2(o[n][2], o[n][3]);
+            } else {
+                *reinterpret_cast<float2*>(row) = make_float2(o[n][0] + o[n][2], o[n][1] + o[n][3]);
+            }
         }
     }
     __syncthreads();
-    // merge the four partial states: warp w finishes query heads g = w, w + 4, ...
-    for (int g = warp; g < G; g += kWarps) {
+    // fold the block's warps into warp 0's slot: element (head, d) belongs to one thread, the statistics are read first
+    for (int e = threadIdx.x; e < G * D; e += kWarps * 32) {
+        const int h = e / D;
         float big = -INFINITY;
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) big = fmaxf(big, s_m[w][g]);
-        float denom = 0.f, num[DPL];
-#pragma unroll
-        for (int d = 0; d < DPL; ++d) num[d] = 0.f;
+        for (int w = 0; w < kWarps; ++w) big = fmaxf(big, st[w * state_floats<D>() + h]);
+        float num = 0.f;
 #pragma unroll
         for (int w = 0; w < kWarps; ++w) {
-            const float f = __expf(s_m[w][g] - big);            // a warp that saw no key holds (-inf, 0, 0): weight 0
-            denom += s_l[w][g] * f;
-#pragma unroll
-            for (int d = 0; d < DPL; ++d) num[d] += s_acc[w][g][lane * DPL + d] * f;
+            const float mw = st[w * state_floats<D>() + h];
+            const float f = mw == -INFINITY ? 0.f : exp2f(mw - big);   // a warp that saw no key: weight 0
+            num += st[w * state_floats<D>() + 2 * kMaxGroup + e] * f;
         }
-        const float inv = 1.f / denom;
-        __nv_bfloat16* o = out + ((long long)b * n_heads + (long long)hk * G + g) * D + lane * DPL;
-#pragma unroll
-        for (int d = 0; d < DPL; d += 2)
-            *reinterpret_cast<uint32_t*>(o + d) = pack_bf16(num[d] * inv, num[d + 1] * inv);
+        st[2 * kMaxGroup + e] = num;
     }
+    __syncthreads();
+    if ((int)threadIdx.x < G) {
+        const int h = threadIdx.x;
+        float big = -INFINITY, den = 0.f;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) big = fmaxf(big, st[w * state_floats<D>() + h]);
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+            const float mw = st[w * state_floats<D>() + h];
+            den += mw == -INFINITY ? 0.f : st[w * state_floats<D>() + kMaxGroup + h] * exp2f(mw - big);
+        }
+        st[h] = big;
+        st[kMaxGroup + h] = den;
+    }
+    __syncthreads();
+    cluster_sync();                                 // every part's state is in its block's shared memory
+    for (int e = 2 * (part * (kWarps * 32) + threadIdx.x); e < G * D; e += 2 * parts * (kWarps * 32)) {
+        const int h = e / D;
+        float big = -INFINITY;
+        for (int c = 0; c < parts; ++c) big = fmaxf(big, ld_cluster(base + 4 * h, c));
+        float den = 0.f, na = 0.f, nb = 0.f;
+        for (int c = 0; c < parts; ++c) {
+            const float mc = ld_cluster(base + 4 * h, c);
+            const float f = mc == -INFINITY ? 0.f : exp2f(mc - big);
+            den += ld_cluster(base + 4 * (kMaxGroup + h), c) * f;
+            na += ld_cluster(base + 4 * (2 * kMaxGroup + e), c) * f;
+            nb += ld_cluster(base + 4 * (2 * kMaxGroup + e + 1), c) * f;
+        }
+        const float inv = 1.f / den;
+        *reinterpret_cast<uint32_t*>(out + ((long long)b * n_heads + (long long)hk * G) * D + e) = pack_bf16(na * inv, nb * inv);
+    }
+    cluster_sync();                                 // nobody leaves while its state is still being read
+}
+
+template <int D, bool SPLIT2>
+static int launch(const void* q, const void* kc, const void* vc, const long long* cols, void* out, int batch, int n_heads,
+                  int n_kv_heads, long long max_len, float scale, int parts, cudaStream_t s) {
+    auto kernel = decode_attention_kernel<D, SPLIT2>;
+    // set for the current device at every launch: the call costs well under a microsecond and keeps no state here
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ring_bytes<D>()) != cudaSuccess) return -10;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)parts, (unsigned)n_kv_heads, (unsigned)batch);
+    cfg.blockDim = dim3(kWarps * 32, 1, 1);
+    cfg.dynamicSmemBytes = ring_bytes<D>();
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)parts;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, (const __nv_bfloat16*)q, (const __nv_bfloat16*)kc,
+                                             (const __nv_bfloat16*)vc, cols, (__nv_bfloat16*)out, n_heads, n_kv_heads, max_len,
+                                             scale, parts);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return -11;
+    }
+    return 0;
 }
 
 }  // namespace decode
@@ -141,17 +370,23 @@ int halo_decode_attention(const void* q, const void* kc, const void* vc, const l
     if (batch < 0 || n_kv_heads < 1 || n_heads % n_kv_heads || n_heads / n_kv_heads > kMaxGroup || max_len < 1) return -1;
     if (head_dim != 128 && head_dim != 64) return -1;
     if (batch == 0) return 0;
-    dim3 grid((unsigned)batch, (unsigned)n_kv_heads);
+    if (batch > 65535 || n_kv_heads > 65535) return -1;
+    if ((reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 15u) return -2;   // 16-byte copies
     cudaStream_t s = (cudaStream_t)stream;
+    // Parts per (sequence, key/value head). The SMs hold 296 blocks, and a part below 128 keys is all merge; up to 4 parts while
+    // the grid stays below two waves (measured at 64 sequences of 8,000 keys: 1 / 2 / 4 / 8 parts 119 / 115 / 106 / 122 us; at
+    // 16 x 4,000: 42 / - / 21 / 27 us). Wider clusters wait for eight free blocks in one GPC at a time and lose, except where
+    // even then no SM gets a second block (2 sequences of 8,000 keys: 4 parts 17.7 us, 8 parts 12.8 us; 16 parts 13.7 us).
+    const long long pairs = (long long)batch * n_kv_heads;
+    const int most = pairs * 8 <= 148 ? 8 : 4;
+    int parts = 1;
+    while (parts < most && pairs * parts < 592 && max_len > 128ll * parts) parts *= 2;
+    const bool split2 = n_heads / n_kv_heads > 8;
     if (head_dim == 128)
-        decode_attention_kernel<4><<<grid, kWarps * 32, 0, s>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)kc,
-                                                                (const __nv_bfloat16*)vc, cols, (__nv_bfloat16*)out, n_heads,
-                                                                n_kv_heads, max_len, scale);
-    else
-        decode_attention_kernel<2><<<grid, kWarps * 32, 0, s>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)kc,
-                                                                (const __nv_bfloat16*)vc, cols, (__nv_bfloat16*)out, n_heads,
-                                                                n_kv_heads, max_len, scale);
-    return cudaGetLastError() == cudaSuccess ? 0 : -11;
+        return split2 ? launch<128, true>(q, kc, vc, cols, out, batch, n_heads, n_kv_heads, max_len, scale, parts, s)
+                      : launch<128, false>(q, kc, vc, cols, out, batch, n_heads, n_kv_heads, max_len, scale, parts, s);
+    return split2 ? launch<64, true>(q, kc, vc, cols, out, batch, n_heads, n_kv_heads, max_len, scale, parts, s)
+                  : launch<64, false>(q, kc, vc, cols, out, batch, n_heads, n_kv_heads, max_len, scale, parts, s);
 }
 
 }  // extern "C"

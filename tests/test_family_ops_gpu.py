@@ -144,6 +144,37 @@ def test_decode_attention_kernel(heads, kv_heads, D):
     assert got.dtype == torch.bfloat16 and (got.float() - want).abs().max() <= 2e-2 * want.abs().max() + 2e-3
 
 
+@pytest.mark.parametrize("B,S,heads,kv_heads,D", [(1, 129, 32, 4, 128), (2, 1100, 32, 4, 128), (37, 530, 24, 2, 128), (40, 1030, 12, 4, 64),
+                                                  (150, 700, 8, 4, 128)])
+def test_decode_attention_parts(B, S, heads, kv_heads, D):
+    """Every split of the keys over blocks (1, 2, 4 and 8 parts, some of them empty), groups above and below eight heads; an
+    infinite value stays infinite. The output is rounded to bf16 once: 2^-8 of the value, plus fp32 noise."""
+    from halo_b200.inference.generate import KVCache
+
+    torch.manual_seed(S)
+    cache = KVCache(1, B, S, kv_heads, D, torch.bfloat16, "cuda")
+    cache.k.normal_()
+    cache.v.normal_()
+    cache.lengths.copy_(torch.randint(0, S, (B,)))
+    cache.lengths[0], cache.lengths[-1] = S - 1, 16
+    cache.v[0, 0, 3, 0, 5] = float("inf")
+    cache.begin_decode()
+    q = torch.randn(B, heads * D, device="cuda").bfloat16()
+    got = cache.attend(0, q, heads).double()
+    ref = KVCache(1, B, S, kv_heads, D, torch.float64, "cuda")
+    ref.k.copy_(cache.k.double())
+    ref.v.copy_(cache.v.double())
+    ref.lengths.copy_(cache.lengths)
+    ref.begin_decode()
+    want = ref.attend(0, q.double(), heads)
+    G = heads // kv_heads
+    first = got[0].view(heads, D)
+    assert torch.isinf(first[:G, 5]).all() and torch.isinf(want[0].view(heads, D)[:G, 5]).all()
+    fine = torch.isfinite(want)
+    assert torch.equal(fine, torch.isfinite(got))
+    assert ((got - want)[fine].abs() <= 2.0 ** -8 * want[fine].abs() + 1e-4).all()
+
+
 def test_generation_on_gpu_matches_teacher_forcing():
     """Greedy sampling through the cache (packed prefill on the flash kernel, decode kernel) against the full forward of
     the grown sequence at every step."""
