@@ -15,6 +15,7 @@
 //
 // Replaces what the reference obtains from cuBLAS (F.linear) and from torch's grouped_mm
 // (halo/kernels/grouped_mm.py:30-51, halo/kernels/expert_gemm.py:14-35).
+#include "gemm_few_rows.cuh"
 #include "gemm_sm100.cuh"
 
 #include <stdio.h>
@@ -654,6 +655,53 @@ static int dispatch_gemm_pair(int a_mn, int b_mn, const CUtensorMap& ta, const C
     return launch_gemm_pair<true, false>(ta, tb, p, n_pairs, s);
 }
 
+// Whether gemm_few_rows_kernel takes a product (both operands K-major, plain store or SwiGLU). The lines follow the table in
+// gemm_few_rows.cuh: up to 16 rows it always wins; above that the tokens' own tiles, which every CTA re-reads from L2, grow
+// with M while the large-tile kernels gain CTAs with N, so wide outputs stay there (`tiles_n`: their tiles along N). Above
+// 128 rows only one CTA fits an SM, which pays where the large tiles leave three quarters of the SMs idle.
+static bool few_rows_wins(int M, int N, int K, int tiles_n, bool glu) {
+    if (M <= 16) return true;
+    if (M <= 64) return tiles_n <= 48;
+    if (M <= 128) return tiles_n <= 32;
+    return M <= 256 && !glu && K >= 4096 && (N + 127) / 128 * 4 <= 148;
+}
+
+static int launch_few_rows(const void* X, const void* W, long long ldx, long long ldw, FewParams p, cudaStream_t stream) {
+    p.m_pad = 16;
+    while (p.m_pad < p.M) p.m_pad *= 2;
+    const int n_tiles = p.swiglu_f ? (p.swiglu_f + 63) / 64 : (p.N + 127) / 128;
+    const int kb = (p.K + kBlockK - 1) / kBlockK;
+    // cut the reduction while the clusters still fit the SMs at once and a part keeps at least 8 blocks of it
+    const int slots = (p.m_pad <= 128 ? 2 : 1) * num_sms(), most = p.m_pad <= 128 ? 8 : 4;
+    p.parts = 1;
+    while (p.parts < most && n_tiles * p.parts * 2 <= slots && kb >= 8 * p.parts) p.parts *= 2;
+    CUtensorMap tw, tx;
+    int rc = make_tmap_bf16(&tx, X, p.M, p.K, ldx, p.m_pad);
+    if (rc) return rc;
+    rc = make_tmap_bf16(&tw, W, p.N, p.K, ldw, p.swiglu_f ? 64 : 128);
+    if (rc) return rc * 10;
+    // the ring also holds the [m_pad][128] fp32 partial sums: m_pad * 512 bytes, less than two stages
+    const int stage_bytes = kFewWBytes + p.m_pad * kBlockK * 2;
+    p.stages = (p.m_pad <= 128 ? 110 : 220) * 1024 / stage_bytes;
+    if (p.stages > kFewMaxStages) p.stages = kFewMaxStages;
+    const int smem = p.stages * stage_bytes + 1024;
+    // set for the current device at every launch (no state is kept here)
+    if (cudaFuncSetAttribute(gemm_few_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -10;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(n_tiles * p.parts), 1, 1);
+    cfg.blockDim = dim3(kFewThreads, 1, 1);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)p.parts;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, gemm_few_rows_kernel, tw, tx, p) == cudaSuccess ? 0 : -11;
+}
+
 // HALO_GEMM_PAIR: 1 (default) = the CTA-pair kernel where it measured faster, 0 = never, 2 = everywhere
 static int g_use_pair = -1;
 static bool use_pair() {
@@ -681,6 +729,16 @@ int halo_gemm_bf16(const void* A, const void* B, void* C, void* aux, int M, int 
     if (M <= 0 || N <= 0 || K < 0) return 0;
     CUtensorMap ta, tb;
     int rc;
+    const bool glu = epi == kEpiSwiglu;
+    if (glu && N % 2) return -20;
+    use_pair();                       // reads HALO_GEMM_PAIR: 2 sends every product to the pair kernel
+    if (g_use_pair != 2 && K > 0 && !a_mn_major && !b_mn_major && (epi == kEpiStoreBf16 || epi == kEpiStoreF32 || glu) &&
+        few_rows_wins(M, N, K, glu ? (N / 2 + 127) / 128 : (N + kBlockN - 1) / kBlockN, glu)) {
+        FewParams f{};
+        f.C = C; f.aux = aux; f.ldc = ldc; f.ld_aux = ld_aux; f.epi = epi; f.alpha = alpha;
+        f.M = M; f.N = N; f.K = K; f.swiglu_f = glu ? N / 2 : 0; f.status = status;
+        return launch_few_rows(A, B, lda, ldb, f, (cudaStream_t)stream);
+    }
     if (a_mn_major) rc = make_tmap_bf16(&ta, A, K, M, lda, 64);
     else rc = make_tmap_bf16(&ta, A, M, K, lda, 128);
     if (rc) return rc;

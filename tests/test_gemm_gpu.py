@@ -51,6 +51,37 @@ def test_matmul_fp32_and_accumulate():
     assert (accb.float() - (1 + ref)).abs().max().item() <= 2e-2 * ref.abs().max().item()
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 128, 64), (3, 136, 200), (16, 4096, 4096), (17, 1000, 776), (64, 2048, 12288), (65, 264, 8200),
+                                   (128, 8192, 512), (129, 4096, 4096), (256, 520, 4104), (257, 264, 4096)])
+def test_few_rows(M, N, K):
+    """Products with few rows at the edges of the dispatch (16, 64, 128 and 256 rows; one to eight cuts of the reduction,
+    ragged N and K): bf16, fp32 and SwiGLU stores into strided outputs against 64-bit sums. fp32 sums of K products of
+    unit normals: the tensor core adds 16 products at a time and cuts the sum to 24 bits, so each of the K / 16 additions
+    loses at most 2 ** -23 of a partial sum that stays below 5 K ** 0.5; bf16 adds 2 ** -8 of the value."""
+    from halo_b200.ops import _lib
+    from halo_b200.ops.gemm import matmul, swiglu_matmul
+
+    torch.manual_seed(M + N)
+    x = torch.randn(M, K + 8, device="cuda").bfloat16()[:, :K]
+    w = torch.randn(N, K, device="cuda").bfloat16()
+    ref = x.double() @ w.double().t()
+    noise = K / 16 * 2.0 ** -23 * 5 * K ** 0.5 + 1e-6
+    out = matmul(x, w, out_dtype=torch.float32, alpha=0.5)
+    assert ((out - 0.5 * ref).abs() <= noise).all()
+    wide = torch.full((M, N + 16), 7.0, dtype=torch.bfloat16, device="cuda")
+    matmul(x, w, out=wide[:, :N])
+    assert ((wide[:, :N] - ref).abs() <= 2.0 ** -8 * ref.abs() + noise).all() and (wide[:, N:] == 7.0).all()
+    scaled = (w.float() * K ** -0.5).bfloat16()
+    F = N // 16 * 8
+    act, pre = swiglu_matmul(x, scaled[:2 * F], save_pre=True)
+    pre_ref = x.double() @ scaled[:2 * F].double().t()
+    assert ((pre - pre_ref).abs() <= 2.0 ** -8 * pre_ref.abs() + 1e-4).all()
+    g, u = pre[:, :F].double(), pre[:, F:].double()
+    act_ref = torch.nn.functional.silu(g) * u
+    assert ((act - act_ref).abs() <= 2.0 ** -7 * act_ref.abs() + 1e-6).all()
+    assert _lib.read_status() == 0
+
+
 def test_swiglu_epilogue():
     from halo_b200.ops.gemm import swiglu_matmul
 
