@@ -250,3 +250,38 @@ def test_rope_attention_fused_matches_reference():
     _close(a.grad.cpu(), b.grad, 4e-2, "dqkv")
     _close(wqa.grad.cpu(), wqb.grad, 5e-2, "dwq")
     _close(wka.grad.cpu(), wkb.grad, 5e-2, "dwk")
+
+
+@pytest.mark.parametrize("T,Hq,Hkv,use_norm,shift", [(1, 2, 1, True, 0), (5, 26, 1, True, 0), (133, 32, 8, True, 0), (4100, 3, 1, True, 0),
+                                                     (33, 8, 4, False, 0), (33, 6, 3, True, 4)])
+def test_qk_norm_rope_head_counts_and_alignment(T, Hq, Hkv, use_norm, shift):
+    """Odd head counts (a pair of heads that straddles q and k, or the end), more heads than one warp takes, more tokens
+    than the fixed backward grid, and rows that start on 8- but not 16-byte boundaries, against 64 bits. Four bf16
+    roundings (2 ** -8 each) of values of at most |x| + |partner|; gradients are rounded once."""
+    from halo_b200.ops.rope import qk_norm_rope, rope_table
+
+    torch.manual_seed(T + Hq)
+    W = (Hq + 2 * Hkv) * 128
+    flat = torch.randn(T * W + shift, device="cuda").bfloat16()
+    qkv = flat[shift:].view(T, W).detach().requires_grad_()
+    wq = (1 + 0.1 * torch.randn(128, device="cuda")).bfloat16().requires_grad_()
+    wk = (1 + 0.1 * torch.randn(128, device="cuda")).bfloat16().requires_grad_()
+    table = rope_table(torch.arange(T, device="cuda"), 128, 1e6)
+    q, k = qk_norm_rope(qkv, wq, wk, table, Hq, Hkv, 1e-6, use_norm)
+    gq, gk = torch.randn_like(q), torch.randn_like(k)
+    leaves = [qkv, wq, wk] if use_norm else [qkv]
+    grads = torch.autograd.grad([q, k], leaves, [gq, gk])
+    xd, wqd, wkd = (t.detach().double().requires_grad_() for t in (qkv, wq, wk))
+    x = xd.view(T, Hq + 2 * Hkv, 128)[:, :Hq + Hkv]
+    if use_norm:
+        w = torch.cat([wqd.expand(Hq, 128), wkd.expand(Hkv, 128)])
+        x = w * (x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + 1e-6))
+    cos, sin = table[:, None, :, 0].double(), table[:, None, :, 1].double()
+    a, b = x[..., :64], x[..., 64:]
+    y = torch.cat([a * cos - b * sin, b * cos + a * sin], -1)
+    bound = 1.02 * 2.0 ** -6 * (x.abs() + torch.cat([b, a], -1).abs()) + 1e-6
+    got = torch.cat([q.view(T, Hq, 128), k.view(T, Hkv, 128)], 1)
+    assert ((got - y).abs() <= bound).all()
+    want = torch.autograd.grad(y, [xd, wqd, wkd] if use_norm else [xd], torch.cat([gq.view(T, Hq, 128), gk.view(T, Hkv, 128)], 1).double())
+    for name, u, v in zip(("dqkv", "dwq", "dwk"), grads, want):
+        assert (u - v).norm() <= 2.0 ** -7 * v.norm() + 1e-6, name
