@@ -54,6 +54,22 @@ def _ce_inplace(logits, labels, grad_scale, row_scale, ignore_index):
     return loss, lse
 
 
+def _scaled_bf16(x, g):
+    """``x`` (fp32 sums or bf16) rounded to bf16 and multiplied by the device scalar ``g``, in one pass."""
+    out = torch.empty(x.shape, dtype=torch.bfloat16, device=x.device)
+    rc = _lib.lib().halo_scale_to_bf16(_lib.ptr(x), _lib.c_int(1 if x.dtype == torch.float32 else 0),
+                                       _lib.ptr(g.reshape(1).to(torch.float32)), _lib.ptr(out), _lib.c_ll(x.numel()),
+                                       _lib.stream_ptr(x.device))
+    _lib.check(rc, "halo_scale_to_bf16")
+    return out
+
+
+def _head_grad_buffer(weight, rows):
+    """fp32 sums of the head's gradient; the first row chunk stores into it, later ones accumulate."""
+    new = torch.empty if rows else torch.zeros
+    return new(weight.shape, dtype=torch.float32, device=weight.device)
+
+
 class _FusedLinearCE(torch.autograd.Function):
     @staticmethod
     def forward(ctx, hidden, weight, labels, grad_scale, chunk_rows, ignore_index):
@@ -63,7 +79,7 @@ class _FusedLinearCE(torch.autograd.Function):
         need_dh = hidden.requires_grad
         need_dw = weight.requires_grad
         dh = torch.empty_like(hidden) if need_dh else None
-        dw32 = torch.zeros((V, H), dtype=torch.float32, device=dev) if need_dw else None
+        dw32 = _head_grad_buffer(weight, T) if need_dw else None
         loss_sum = torch.zeros((), dtype=torch.float32, device=dev)
         Vp = (V + 7) // 8 * 8
         buf = torch.empty((min(chunk_rows, max(T, 1)), Vp), dtype=torch.bfloat16, device=dev)
@@ -77,19 +93,18 @@ class _FusedLinearCE(torch.autograd.Function):
             if need_dh:
                 matmul(logits, weight, b_t=False, out=dh[s:e])
             if need_dw:
-                matmul(logits, hc, a_t=True, b_t=False, out=dw32, accumulate=True)
-        ctx.save_for_backward(dh, dw32.to(weight.dtype) if need_dw else None)
+                matmul(logits, hc, a_t=True, b_t=False, out=dw32, accumulate=s > 0)
+        ctx.save_for_backward(dh, dw32)
         return loss_sum * grad_scale
-
 
     @staticmethod
     def backward(ctx, g):
         dh, dw = ctx.saved_tensors
         # the stored gradients already carry grad_scale; g is the upstream scalar (1 for a plain loss)
         if dh is not None:
-            dh = dh * g.to(dh.dtype)
+            dh = _scaled_bf16(dh, g)
         if dw is not None:
-            dw = dw * g.to(dw.dtype)
+            dw = _scaled_bf16(dw, g)
         return dh, dw, None, None, None, None
 
 
@@ -158,7 +173,7 @@ class _LinearLogprobs(torch.autograd.Function):
         V = weight.shape[0]
         dev = hidden.device
         dh = torch.empty_like(hidden) if ctx.needs_input_grad[0] else None
-        dw32 = torch.zeros((V, H), dtype=torch.float32, device=dev) if ctx.needs_input_grad[1] else None
+        dw32 = _head_grad_buffer(weight, T) if ctx.needs_input_grad[1] else None
         Vp = (V + 7) // 8 * 8
         buf = torch.empty((min(chunk_rows, max(T, 1)), Vp), dtype=torch.bfloat16, device=dev)
         neg = (-g_logp).to(torch.float32).contiguous()
@@ -171,7 +186,7 @@ class _LinearLogprobs(torch.autograd.Function):
             if dh is not None:
                 matmul(logits, weight, b_t=False, out=dh[s:e])
             if dw32 is not None:
-                matmul(logits, hidden[s:e], a_t=True, b_t=False, out=dw32, accumulate=True)
+                matmul(logits, hidden[s:e], a_t=True, b_t=False, out=dw32, accumulate=s > 0)
         return dh, (dw32.to(weight.dtype) if dw32 is not None else None), None, None, None, None
 
 

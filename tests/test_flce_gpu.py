@@ -47,3 +47,33 @@ def test_linear_logprobs():
     assert (ent - ent_ref).abs().max().item() <= 5e-2
     assert (ha.grad.float() - hb.grad).abs().max().item() <= 5e-2 * hb.grad.abs().max().item() + 1e-6
     assert (wa.grad.float() - wb.grad).abs().max().item() <= 5e-2 * wb.grad.abs().max().item() + 1e-6
+
+
+@pytest.mark.parametrize("T,V,chunk", [(129, 4104, 128), (3, 264, 4096), (7, 40960, 4)])
+def test_head_loss_edges_and_upstream_scale(T, V, chunk):
+    """Row chunks of one row, vector remainders of the row kernels, all rows of a chunk ignored, and an upstream gradient
+    that is not 1, against 64-bit sums over the bf16 logits' own rounding (2 ** -8 of a logit of up to 5 moves a
+    log-probability by that much; the stored gradients are rounded to bf16 twice)."""
+    from halo_b200.ops.cross_entropy import fused_linear_cross_entropy, linear_logprobs
+
+    torch.manual_seed(T)
+    H = 128
+    h = torch.randn(T, H, device="cuda").bfloat16().requires_grad_()
+    w = (torch.randn(V, H, device="cuda") * H ** -0.5).bfloat16().requires_grad_()
+    labels = torch.randint(0, V, (T,), device="cuda")
+    labels[0] = V - 1
+    labels[-1] = -100
+    loss = fused_linear_cross_entropy(h, w, labels, chunk_rows=chunk)
+    dh, dw = torch.autograd.grad(3.0 * loss, [h, w], retain_graph=True)
+    again = torch.autograd.grad(3.0 * loss, [h, w])
+    assert torch.equal(dh, again[0]) and torch.equal(dw, again[1])      # the stored gradients are not consumed
+    hd, wd = h.detach().double().requires_grad_(), w.detach().double().requires_grad_()
+    z = hd @ wd.t()
+    ref = torch.nn.functional.cross_entropy(z, labels, ignore_index=-100)
+    (3.0 * ref).backward()
+    assert abs(loss.item() - ref.item()) <= 2.0 ** -8 * ref.item()
+    assert (dh - hd.grad).norm() <= 2.0 ** -6 * hd.grad.norm() and (dw - wd.grad).norm() <= 2.0 ** -6 * wd.grad.norm()
+    logp, ent = linear_logprobs(h.detach(), w.detach(), labels, chunk_rows=chunk, want_entropy=True)
+    lp = torch.log_softmax(z.detach(), -1)
+    want = torch.where(labels == -100, 0.0, lp.gather(-1, labels.clamp_min(0)[:, None])[:, 0])
+    assert (logp - want).abs().max() <= 2.0 ** -8 * 5 and (ent + (lp.exp() * lp).sum(-1)).abs().max() <= 2.0 ** -8 * 5
