@@ -54,18 +54,9 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], 
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ float ld_cluster(uint32_t local_addr, uint32_t rank) {
-    uint32_t a;
     float v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local_addr), "r"(rank));
+    const uint32_t a = map_to_cta(local_addr, rank);
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
     return v;
 }
@@ -90,7 +81,7 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
     constexpr int kTile = kTileKeys * kRow;         // bytes of a warp's key (or value) tile
     constexpr int kChunks = D / 8;                  // 16-byte chunks per row
     const int b = blockIdx.z, hk = blockIdx.y;
-    const uint32_t part = cluster_rank();
+    const uint32_t part = cluster_cta_rank();
     const int G = n_heads / n_kv_heads;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;          // fragment row and column pair of this lane
@@ -310,7 +301,7 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
         st[kMaxGroup + h] = den;
     }
     __syncthreads();
-    cluster_sync();                                 // every part's state is in its block's shared memory
+    cluster_sync_all();                                 // every part's state is in its block's shared memory
     for (int e = 2 * (part * (kWarps * 32) + threadIdx.x); e < G * D; e += 2 * parts * (kWarps * 32)) {
         const int h = e / D;
         float big = -INFINITY;
@@ -326,7 +317,7 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
         const float inv = 1.f / den;
         *reinterpret_cast<uint32_t*>(out + ((long long)b * n_heads + (long long)hk * G) * D + e) = pack_bf16(na * inv, nb * inv);
     }
-    cluster_sync();                                 // nobody leaves while its state is still being read
+    cluster_sync_all();                                 // nobody leaves while its state is still being read
 }
 
 template <int D, bool SPLIT2>

@@ -46,18 +46,9 @@ struct FewParams {
     int* status;
 };
 
-__device__ __forceinline__ uint32_t few_cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void few_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ float2 ld_cluster_f2(uint32_t local_addr, uint32_t rank) {
-    uint32_t a;
     float2 v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local_addr), "r"(rank));
+    const uint32_t a = map_to_cta(local_addr, rank);
     asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
     return v;
 }
@@ -71,7 +62,7 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
     __shared__ volatile int abort_flag;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t rank = few_cluster_rank();
+    const uint32_t rank = cluster_cta_rank();
     const int tile = blockIdx.x / p.parts;
     const int stage_bytes = kFewWBytes + p.m_pad * kBlockK * 2;
     const int tmem_cols = p.m_pad < 32 ? 32 : p.m_pad;
@@ -158,7 +149,7 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
         }
     }
     __syncthreads();
-    if (p.parts > 1) few_cluster_sync();            // every CTA's partial sums are in place
+    if (p.parts > 1) cluster_sync_all();            // every CTA's partial sums are in place
 
     if (warp >= 2 && !abort_flag) {
         // thread t of the four warps owns two neighbouring columns of every second token of this CTA's share
@@ -211,7 +202,7 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
         while (global_timer_ns() - t0 < 2000000ull) { }
         __syncthreads();
     }
-    if (p.parts > 1) few_cluster_sync();            // nobody leaves while its partial sums are still being read
+    if (p.parts > 1) cluster_sync_all();            // nobody leaves while its partial sums are still being read
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem, tmem_cols);

@@ -65,6 +65,7 @@ struct GemmParams {
     // NVLink stores of the early tiles drain while the later tiles are still being multiplied.
     void* c_peers[8];
     int rs_ranks, rs_rank, rs_rows;
+    int wide_full, wide_items;   // gemm_wide_kernel, dense: whole tiles, and work items with the column halves that follow them
     // kEpiClampedGlu: bias bank as one bf16 vector indexed like the rows of B, the clamp and the gate's slope
     const void* glu_bias;
     float glu_limit, glu_alpha;

@@ -265,14 +265,24 @@ def _alloc(transport, shape, dtype, dev):
 _PAIR_ENABLED = None
 
 
-def _pair_ok(k_dim: int, swiglu: bool) -> int:
-    """Which GEMM kernel runs a grouped product. On the 30B-A3B expert shapes the CTA-pair form (256-row tiles)
-    shortens the kernels themselves by only 1-5 % and the step as a whole measured no faster, so grouped products
-    stay on the single-CTA kernel unless HALO_GEMM_PAIR=2 forces the pair form everywhere."""
+def _pair_mode() -> int:
     global _PAIR_ENABLED
     if _PAIR_ENABLED is None:
         _PAIR_ENABLED = int(_lib.lib().halo_gemm_pair_enabled())
-    return int(_PAIR_ENABLED == 2 and not swiglu)
+    return _PAIR_ENABLED
+
+
+def _pair_ok(k_dim: int, swiglu: bool) -> int:
+    """Which GEMM kernel runs a product over an expert's rows: the single-CTA kernel (128-row tiles, the padding of a segment)
+    unless HALO_GEMM_PAIR=2 forces the CTA-pair form (256 x 512 tiles) everywhere."""
+    return int(_pair_mode() == 2 and not swiglu)
+
+
+def _pair_weight_grads() -> int:
+    """The weight-gradient products reduce over an expert's rows and tile the bank itself, which has no ragged edge in rows: they
+    run on the CTA-pair kernel (65,536 tokens of the 30B-A3B shapes: 5,591 us on the single-CTA kernel, 5,192 us; 3,001 tokens
+    546 and 505 us) unless HALO_GEMM_PAIR=0."""
+    return int(_pair_mode() != 0)
 
 
 def _tile_list(state: RoutingState, kind: str, pair: int = 0, **kw):
@@ -607,7 +617,7 @@ def _fused_backward(ctx, dout):
     dw_gate_up = dw_down = None
     if ctx.needs_input_grad[3] or ctx.needs_input_grad[4]:
         dw_down = _alloc(transport, tuple(w_down.shape), w_down.dtype, dev)
-        pk = _pair_ok(4096, False)
+        pk = _pair_weight_grads()
         _gemm_list(dy, act_w, dw_down.reshape(E_local * H, F), _tile_list(state, "k", pk, m_dim=H, n_dim=F), 1, 1,
                    EPI_STORE_BF16, pair=pk)
         dw_gate_up = _alloc(transport, tuple(w_gate_up.shape), w_gate_up.dtype, dev)
@@ -779,7 +789,7 @@ class _MoEExperts(torch.autograd.Function):
                 return None, None
             # 5. dW_down[e] = dout_e^T (w * act)_e ; dW_gate_up[e] = dpre_e^T x_e
             dw_down = _alloc(transport, tuple(w_down.shape), w_down.dtype, dev)
-            pk = _pair_ok(4096, False)      # the reduction runs over an expert's rows: long
+            pk = _pair_weight_grads()
             _gemm_list(dy, act_w, dw_down.reshape(E_local * H, F), _tile_list(state, "k", pk, m_dim=H, n_dim=F), 1, 1,
                        EPI_STORE_BF16, pair=pk)
             dw_gate_up = _alloc(transport, tuple(w_gate_up.shape), w_gate_up.dtype, dev)

@@ -82,6 +82,40 @@ def test_few_rows(M, N, K):
     assert _lib.read_status() == 0
 
 
+@pytest.mark.parametrize("M,N,K", [(5000, 4104, 64), (9001, 776, 136), (20000, 264, 200), (2500, 6000, 256), (19000, 520, 328)])
+def test_wide_tiles(M, N, K):
+    """The 256 x 512 pair tiles at their edges: one to six blocks of the reduction (the second column block starts up to three
+    late), ragged rows and columns, a last wave cut into column halves, every operand layout, stores and accumulation in
+    both types, SwiGLU. Bounds as for the few-row products."""
+    from halo_b200.ops import _lib
+    from halo_b200.ops.gemm import matmul, swiglu_matmul
+
+    torch.manual_seed(N)
+    noise = K / 16 * 2.0 ** -23 * 5 * K ** 0.5 + 1e-6
+    m8 = (M + 7) // 8 * 8
+    for a_t in (False, True):
+        a = torch.randn((K, m8) if a_t else (M, K), device="cuda").bfloat16()
+        a = a[:, :M] if a_t else a
+        for b_t in (False, True):
+            b = torch.randn((N, K) if b_t else (K, N), device="cuda").bfloat16()
+            ref = (a.double().t() if a_t else a.double()) @ (b.double().t() if b_t else b.double())
+            out = torch.full((M, N), 2.0, device="cuda")
+            matmul(a, b, a_t=a_t, b_t=b_t, out=out, accumulate=True, alpha=0.5)
+            assert ((out - 2.0 - 0.5 * ref).abs() <= noise + 2.0 ** -22 * (ref.abs() + 4)).all()
+            wide = torch.full((M, N + 8), 7.0, dtype=torch.bfloat16, device="cuda")
+            matmul(a, b, a_t=a_t, b_t=b_t, out=wide[:, :N])
+            assert ((wide[:, :N] - ref).abs() <= 2.0 ** -8 * ref.abs() + noise).all() and (wide[:, N:] == 7.0).all()
+            matmul(a, b, a_t=a_t, b_t=b_t, out=wide[:, :N], accumulate=True)
+            assert ((wide[:, :N] - 2 * ref).abs() <= 3 * 2.0 ** -8 * ref.abs() * 1.5 + 2 * noise).all()
+    x, w = torch.randn(M, K, device="cuda").bfloat16(), (torch.randn(2 * N, K, device="cuda") * K ** -0.5).bfloat16()
+    act, pre = swiglu_matmul(x, w, save_pre=True)
+    pre_ref = x.double() @ w.double().t()
+    assert ((pre - pre_ref).abs() <= 2.0 ** -8 * pre_ref.abs() + 1e-4).all()
+    act_ref = torch.nn.functional.silu(pre[:, :N].double()) * pre[:, N:].double()
+    assert ((act - act_ref).abs() <= 2.0 ** -7 * act_ref.abs() + 1e-6).all()
+    assert torch.equal(swiglu_matmul(x, w)[0], act) and _lib.read_status() == 0
+
+
 def test_swiglu_epilogue():
     from halo_b200.ops.gemm import swiglu_matmul
 
