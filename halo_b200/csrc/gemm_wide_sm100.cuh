@@ -248,6 +248,8 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_slot;
 
+    // Every role reads its next item before it works on this one: a listed item comes from L2 or HBM, and the wait for it would
+    // otherwise drain the tensor pipe between tiles.
     const int total = p.list ? *p.list_count : p.wide_items;
     const int first = blockIdx.x >> 1, step = gridDim.x >> 1;
 
@@ -256,8 +258,11 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (lane == 0) {
             int stage = 0;
             uint32_t phase = 0;
-            GemmWork w;
-            for (int idx = first; wide_fetch(p, idx, total, w) && !abort_flag; idx += step) {
+            GemmWork w, next;
+            bool more = wide_fetch(p, first, total, next);
+            for (int idx = first + step; more && !abort_flag; idx += step) {
+                w = next;
+                more = wide_fetch(p, idx, total, next);
                 const int a_mn = w.a_mn + int(rank) * 128;
                 for (int kb = 0; kb < w.k_iters; ++kb) {
                     if (!mbar_wait(smem_u32(&bar_empty[stage]), phase ^ 1u, &abort_flag, p.status)) break;
@@ -293,7 +298,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             constexpr uint32_t idesc = make_idesc_bf16(256, kBlockN, A_MN ? 1 : 0, B_MN ? 1 : 0);
             int stage = 0;
             uint32_t phase = 0, used[2] = {0, 0};       // tiles each accumulator block has served
-            GemmWork w;
+            GemmWork w, next;
             auto issue = [&](int s, int block, bool accumulate) {
                 const uint32_t sa = tiles_base + s * kWideStageBytes, sb = sa + (1 + block) * kATileBytes;
 #pragma unroll
@@ -303,7 +308,10 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                     wide_mma(tmem_base + block * kBlockN, da, db, idesc, (accumulate || k) ? 1u : 0u);
                 }
             };
-            for (int idx = first; wide_fetch(p, idx, total, w) && !abort_flag; idx += step) {
+            bool more = wide_fetch(p, first, total, next);
+            for (int idx = first + step; more && !abort_flag; idx += step) {
+                w = next;
+                more = wide_fetch(p, idx, total, next);
                 if (!mbar_wait(smem_u32(&bar_tempty[0]), (used[0] & 1u) ^ 1u, &abort_flag, p.status)) break;
                 tc_fence_after();
                 ++used[0];
@@ -362,7 +370,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const bool f32 = p.epi == kEpiStoreF32 || p.epi == kEpiAccumF32;
         const bool wide_values = f32 || p.epi == kEpiAccumBf16;
         uint32_t used[2] = {0, 0};
-        GemmWork w;
+        GemmWork w, next;
         auto ready = [&](int block) -> bool {            // the block's products are complete
             if (!mbar_wait(smem_u32(&bar_tfull[block]), used[block]++ & 1u, &abort_flag, p.status)) return false;
             tc_fence_after();
@@ -373,7 +381,10 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             __syncwarp();
             if (lane == 0) mbar_arrive_remote(map_to_cta(smem_u32(&bar_tempty[block]), 0));
         };
-        for (int idx = first; wide_fetch(p, idx, total, w) && !abort_flag; idx += step) {
+        bool more = wide_fetch(p, first, total, next);
+        for (int idx = first + step; more && !abort_flag; idx += step) {
+            w = next;
+            more = wide_fetch(p, idx, total, next);
             const int rows = max(0, min(32, w.m_valid - int(rank) * 128 - row0));       // rows of this warp that exist
             const long long c_row = (long long)w.c_row + int(rank) * 128 + row0;
             const bool zero = w.k_iters == 0;

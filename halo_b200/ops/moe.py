@@ -280,8 +280,8 @@ def _pair_ok(k_dim: int, swiglu: bool) -> int:
 
 def _pair_weight_grads() -> int:
     """The weight-gradient products reduce over an expert's rows and tile the bank itself, which has no ragged edge in rows: they
-    run on the CTA-pair kernel (65,536 tokens of the 30B-A3B shapes: 5,591 us on the single-CTA kernel, 5,192 us; 3,001 tokens
-    546 and 505 us) unless HALO_GEMM_PAIR=0."""
+    run on the CTA-pair kernel (the 30B-A3B shapes, gate_up + down: 65,536 tokens with uneven loads 3,096 + 1,627 us on the
+    single-CTA kernel and 2,817 + 1,583 us on this one, 3,001 tokens 389 + 226 and 341 + 187 us) unless HALO_GEMM_PAIR=0."""
     return int(_pair_mode() != 0)
 
 
@@ -340,8 +340,9 @@ def grouped_swiglu_ffn_fwd(state: RoutingState, x_rows, w_gate_up, w_down, save_
     dev = x_rows.device
     act = _alloc(transport, (cap, F), torch.bfloat16, dev)
     pre = _alloc(transport, (cap, F2), torch.bfloat16, dev) if save_pre else None
-    lst1 = _tile_list(state, "m", n_cols=F2, k_dim=H, b_mn_stride=F2, b_k_stride=0, swiglu_f=F)
-    _gemm_list(x_rows, w_gate_up.reshape(E * F2, H), act, lst1, 0, 0, EPI_SWIGLU, aux=pre, swiglu_f=F)
+    pair = _pair_ok(H, False)
+    lst1 = _tile_list(state, "m", pair, n_cols=F2, k_dim=H, b_mn_stride=F2, b_k_stride=0, swiglu_f=F)
+    _gemm_list(x_rows, w_gate_up.reshape(E * F2, H), act, lst1, 0, 0, EPI_SWIGLU, aux=pre, swiglu_f=F, pair=pair)
     return act, pre
 
 

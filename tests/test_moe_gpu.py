@@ -195,3 +195,40 @@ def test_router_topk_selection_bias_matches_reference():
     assert torch.equal(idx.sort(-1).values, ridx.sort(-1).values)
     assert torch.allclose(w.sum(-1), torch.ones_like(w.sum(-1)), atol=1e-5)
     assert torch.allclose(w.sort(-1).values, rw.sort(-1).values, atol=1e-5)
+
+
+@pytest.mark.parametrize("pair", [0, 1])
+@pytest.mark.parametrize("E,T,H,F", [(3, 900, 520, 264), (130, 700, 256, 768), (16, 3000, 1032, 512)])
+def test_grouped_products_over_uneven_experts(pair, E, T, H, F):
+    """Every form of grouped product on both GEMM kernels - rows grouped along the output and along the reduction - with
+    empty experts, one that holds half of the rows and ragged column tiles: each tile of the longest-first list is visited
+    once (fp32 sums of at most 1,500 products, rounded to bf16)."""
+    from halo_b200.ops import _lib, moe
+
+    torch.manual_seed(E)
+    weights = torch.rand(E, device="cuda")
+    weights[1] = 0.0
+    weights[2] = weights.sum()
+    idx = torch.multinomial(weights.expand(T, E), 2).int() if E > 3 else torch.where(torch.rand(T, 2, device="cuda") < 0.5, 0, 2).int()
+    state = moe.plan_routing(idx, E, moe.LocalTransport())
+    cap = state.capacity
+    x = torch.zeros(cap, H, device="cuda", dtype=torch.bfloat16)
+    y = torch.zeros(cap, F, device="cuda", dtype=torch.bfloat16)
+    starts, rows = state.seg_start.tolist(), state.seg_rows.tolist()
+    assert 0 in rows
+    for s, n in zip(starts, rows):
+        x[s:s + n].normal_()
+        y[s:s + n].normal_()
+    out = torch.full((E, F, H), 7.0, device="cuda", dtype=torch.bfloat16)
+    moe._gemm_list(y, x, out.view(E * F, H), moe._tile_list(state, "k", pair, m_dim=F, n_dim=H), 1, 1, 0, pair=pair)
+    w = (torch.randn(E, H, F, device="cuda") * F ** -0.5).bfloat16()
+    z = torch.full((cap, H), 7.0, device="cuda", dtype=torch.bfloat16)
+    moe._gemm_list(y, w.view(E * H, F), z, moe._tile_list(state, "m", pair, n_cols=H, k_dim=F, b_mn_stride=H, b_k_stride=0, swiglu_f=0),
+                   0, 0, 0, pair=pair)
+    for e, (s, n) in enumerate(zip(starts, rows)):
+        want = y[s:s + n].double().t() @ x[s:s + n].double()
+        assert ((out[e] - want).abs() <= 2.0 ** -8 * want.abs() + 1e-3).all(), e
+        want = y[s:s + n].double() @ w[e].double().t()
+        assert ((z[s:s + n] - want).abs() <= 2.0 ** -8 * want.abs() + 1e-3).all(), e
+        assert (z[s + n:s + (n + 127) // 128 * 128] == 0).all()
+    assert _lib.read_status() == 0
