@@ -149,3 +149,27 @@ def test_adamw_q8_kernel_equals_its_tensor_op_statement(grad_dtype):
     og.arm_skip(skip)
     og.step()
     assert all(torch.equal(a, pg) for a, (_, pg) in zip(before, gpu))
+
+
+@pytest.mark.parametrize("numel,offset", [(7, 0), (16384, 0), (16385, 8), (40000, 1), (50003, 4)])
+def test_adamw_blocks_and_alignment(numel, offset):
+    """Whole blocks, the ragged last one and tensors off the 16-byte boundary, with zero and overflowing gradients, bit
+    for bit against the CPU statement."""
+    from halo_b200.optim.adamw_bf16 import AdamWBF16, adamw_bf16_step_reference, param_name_hash
+
+    gen = torch.Generator().manual_seed(numel)
+    flat = torch.randn(numel + offset, generator=gen).bfloat16()
+    grad = (torch.randn(numel, generator=gen) * torch.logspace(-30, 18, numel)[torch.randperm(numel, generator=gen)]).bfloat16()
+    grad[0], grad[1] = 0.0, 3e38      # the second moment overflows to infinity: the update is then zero
+    p = torch.nn.Parameter(flat.cuda()[offset:])
+    opt = AdamWBF16([("w", p)], lr=1e-2)
+    pc, mc, vc = flat[offset:].clone(), torch.zeros(numel).bfloat16(), torch.zeros(numel).bfloat16()
+    for step in (1, 2, 3):
+        p.grad = grad.cuda()
+        opt.step()
+        adamw_bf16_step_reference(pc, grad, mc, vc, beta1=0.9, beta2=0.999, step_size=1e-2 / (1 - 0.9 ** step),
+                                  bc2_sqrt=(1 - 0.999 ** step) ** 0.5, eps=1e-8, wd_factor=1 - 1e-2 * 0.01, key=opt.key, step=step,
+                                  name_hash=param_name_hash("w"))
+        for got, want in ((p, pc), (opt.state[p]["exp_avg"], mc), (opt.state[p]["exp_avg_sq"], vc)):
+            got = got.detach().cpu()
+            assert torch.equal(got.view(torch.int16), want.view(torch.int16))
