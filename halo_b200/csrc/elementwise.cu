@@ -316,18 +316,36 @@ __device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
     return *reinterpret_cast<const uint32_t*>(&r);
 }
 
-template <bool A16>
+// CACHE (sampling): the rotated keys and the values also go to their places in a key/value cache, so that a step needs no
+// scatter of its own (two index_put launches a layer before).
+struct RopeCache {
+    __nv_bfloat16* k;            // one layer's cache, [batch, max_len, Hkv, 128]
+    __nv_bfloat16* v;
+    const long long* rows;       // [T] sequence and position of every token
+    const long long* cols;
+    long long batch, max_len;
+    int* status;
+};
+
+template <bool A16, bool CACHE>
 __global__ void __launch_bounds__(256)
 qknorm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __restrict__ wq,
                        const __nv_bfloat16* __restrict__ wk, const float2* __restrict__ table,
                        __nv_bfloat16* __restrict__ q_out, __nv_bfloat16* __restrict__ k_out,
-                       float* __restrict__ rstd_out, long long T, int Hq, int Hkv, float eps, int use_norm, int splits) {
+                       float* __restrict__ rstd_out, long long T, int Hq, int Hkv, float eps, int use_norm, int splits,
+                       const RopeCache cache) {
     const int lane = threadIdx.x & 31, l16 = lane & 15, which = lane >> 4;
     const long long wid = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (wid >= T * splits) return;
     const long long t = wid / splits;
-    const int heads = Hq + Hkv;
+    const int rotated = Hq + Hkv, heads = CACHE ? rotated + Hkv : rotated;
     const int pair0 = (int)(wid % splits) * kRopePairs;
+    long long place = -1;        // this token's first cached element
+    if (CACHE) {
+        const long long r = cache.rows[t], c = cache.cols[t];
+        if (r >= 0 && r < cache.batch && c >= 0 && c < cache.max_len) place = (r * cache.max_len + c) * Hkv * 128 + l16 * 8;
+        else if (lane == 0 && cache.status) atomicCAS(cache.status, kStatusOk, kStatusBounds);
+    }
     const __nv_bfloat16* src = qkv + t * (long long)(Hq + 2 * Hkv) * 128 + l16 * 8;
     uint4 raw[kRopePairs];
 #pragma unroll
@@ -357,7 +375,7 @@ qknorm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat1
             for (int j = 0; j < 8; ++j) ss += v[j] * v[j];
             ss = half_warp_sum(ss);
             const float rstd = rsqrtf(ss / 128.f + eps);
-            if (l16 == 0 && live) rstd_out[t * heads + hd] = rstd;
+            if (l16 == 0 && rstd_out && hd < rotated) rstd_out[t * rotated + hd] = rstd;
             const uint4 w = is_q ? wqv : wkv;
             const uint32_t wp[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
@@ -372,9 +390,13 @@ qknorm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat1
             const float2 x = unpack2(n[j]), y = unpack2(partner);
             o[j] = add_bf16x2(pack_bf16(x.x * cs[2 * j], x.y * cs[2 * j + 1]), pack_bf16(y.x * sn[2 * j], y.y * sn[2 * j + 1]));
         }
-        if (live) {
-            __nv_bfloat16* dst = is_q ? q_out + (t * Hq + hd) * 128 + l16 * 8 : k_out + (t * Hkv + (hd - Hq)) * 128 + l16 * 8;
-            store8<A16>(dst, out);
+        if (is_q) {
+            store8<A16>(q_out + (t * Hq + hd) * 128 + l16 * 8, out);
+        } else if (hd < rotated) {
+            if (k_out) store8<A16>(k_out + (t * Hkv + (hd - Hq)) * 128 + l16 * 8, out);
+            if (CACHE && place >= 0) store8<A16>(cache.k + place + (long long)(hd - Hq) * 128, out);
+        } else if (CACHE && live && place >= 0) {
+            store8<A16>(cache.v + place + (long long)(hd - rotated) * 128, raw[i]);       // values are stored as they are
         }
     }
 }
@@ -889,11 +911,30 @@ int halo_qknorm_rope_fwd(const void* qkv, const void* wq, const void* wk, const 
     const int splits = rope_splits(Hq + Hkv);
     const unsigned grid = (unsigned)((T * splits + 7) / 8);
     const bool a16 = (((uintptr_t)qkv | (uintptr_t)q_out | (uintptr_t)k_out | (uintptr_t)table) & 15u) == 0;
-    auto kernel = a16 ? qknorm_rope_fwd_kernel<true> : qknorm_rope_fwd_kernel<false>;
+    auto kernel = a16 ? qknorm_rope_fwd_kernel<true, false> : qknorm_rope_fwd_kernel<false, false>;
     kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(
         (const __nv_bfloat16*)qkv, (const __nv_bfloat16*)wq, (const __nv_bfloat16*)wk,
         (const float2*)table, (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_out, rstd, T, Hq, Hkv, eps,
-        use_norm, splits);
+        use_norm, splits, RopeCache{});
+    return HALO_LAUNCH_CHECK();
+}
+
+// As halo_qknorm_rope_fwd without the statistics, for sampling: the rotated keys and the values go to places (rows[t], cols[t])
+// of one layer's cache [batch, max_len, Hkv, 128]; k_out may be null. A place outside the cache is skipped and recorded.
+int halo_qknorm_rope_cache(const void* qkv, const void* wq, const void* wk, const void* table, void* q_out, void* k_out,
+                           void* k_cache, void* v_cache, const long long* rows, const long long* cols, long long batch,
+                           long long max_len, long long T, int Hq, int Hkv, int head_dim, float eps, int use_norm, int* status,
+                           void* stream) {
+    if (head_dim != 128) return -1;
+    const int splits = rope_splits(Hq + 2 * Hkv);
+    const unsigned grid = (unsigned)((T * splits + 7) / 8);
+    const bool a16 = (((uintptr_t)qkv | (uintptr_t)q_out | (uintptr_t)k_out | (uintptr_t)table | (uintptr_t)k_cache |
+                       (uintptr_t)v_cache) & 15u) == 0;
+    auto kernel = a16 ? qknorm_rope_fwd_kernel<true, true> : qknorm_rope_fwd_kernel<false, true>;
+    const RopeCache cache{(__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, rows, cols, batch, max_len, status};
+    kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(
+        (const __nv_bfloat16*)qkv, (const __nv_bfloat16*)wq, (const __nv_bfloat16*)wk, (const float2*)table,
+        (__nv_bfloat16*)q_out, (__nv_bfloat16*)k_out, nullptr, T, Hq, Hkv, eps, use_norm, splits, cache);
     return HALO_LAUNCH_CHECK();
 }
 

@@ -104,6 +104,34 @@ class KVCache:
         self.v[li][self._rows, self._cols] = v.reshape(-1, Hkv, D)
         return li
 
+    def rotate_and_write(self, qkv, attn, table, keep_keys: bool):
+        """q / k norm, rotary embedding and the cache write of this layer in one kernel, or None where it does not apply (then
+        :func:`qk_norm_rope` and :meth:`write` do). Returns ``(q, k or None, layer index)``."""
+        cfg = attn.cfg
+        Hq, Hkv, D = cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim
+        wq, wk = attn.q_norm, attn.k_norm
+        if (not qkv.is_cuda or D != 128 or qkv.dtype != torch.bfloat16 or self.k.dtype != torch.bfloat16 or 2 * table.shape[1] != D
+                or tuple(self.k.shape[-2:]) != (Hkv, D) or qkv.shape[1] != (Hq + 2 * Hkv) * D or self._rows.dtype != torch.long
+                or self._cols.dtype != torch.long or (cfg.use_qk_norm and (wq is None or wq.numel() != D))
+                or (torch.is_grad_enabled() and qkv.requires_grad) or qkv.shape[0] == 0):
+            return None
+        from halo_b200.ops import _lib
+
+        li = self._layer
+        self._layer += 1
+        qkv = qkv.contiguous()
+        T, dev = qkv.shape[0], qkv.device
+        q = torch.empty((T, Hq * D), dtype=torch.bfloat16, device=dev)
+        k = torch.empty((T, Hkv * D), dtype=torch.bfloat16, device=dev) if keep_keys else None
+        rows, cols = self._rows.contiguous(), self._cols.contiguous()
+        rc = _lib.lib().halo_qknorm_rope_cache(
+            _lib.ptr(qkv), _lib.ptr(wq), _lib.ptr(wk), _lib.ptr(table), _lib.ptr(q), _lib.ptr(k), _lib.ptr(self.k[li]),
+            _lib.ptr(self.v[li]), _lib.ptr(rows), _lib.ptr(cols), _lib.c_ll(self.k.shape[1]), _lib.c_ll(self.k.shape[2]),
+            _lib.c_ll(T), _lib.c_int(Hq), _lib.c_int(Hkv), _lib.c_int(D), _lib.c_float(cfg.rms_norm_eps),
+            _lib.c_int(1 if cfg.use_qk_norm else 0), _lib.ptr(_lib.status_word(dev)), _lib.stream_ptr(dev))
+        _lib.check(rc, "halo_qknorm_rope_cache")
+        return q, k, li
+
     def attend(self, li: int, q: torch.Tensor, n_heads: int, scale: float | None = None, window: int = 0,
                sinks: torch.Tensor | None = None, softcap: float = 0.0) -> torch.Tensor:
         """One query per sequence ``[B, heads * head_dim]`` against keys ``0 .. lengths[b]`` (the token just written
@@ -152,9 +180,13 @@ def cached_attention(attn, h, ctx):
     cfg, cache = attn.cfg, ctx.kv_cache
     Hq, Hkv, D = cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim
     qkv = attn._qkv(h)
-    q, k = qk_norm_rope(qkv, attn.q_norm, attn.k_norm, attn.rope_of(ctx), Hq, Hkv, cfg.rms_norm_eps, cfg.use_qk_norm)
     v = qkv[:, (Hq + Hkv) * D:]
-    li = cache.write(k, v)
+    done = cache.rotate_and_write(qkv, attn, attn.rope_of(ctx), keep_keys=cache.mode == "prefill")
+    if done is not None:
+        q, k, li = done
+    else:
+        q, k = qk_norm_rope(qkv, attn.q_norm, attn.k_norm, attn.rope_of(ctx), Hq, Hkv, cfg.rms_norm_eps, cfg.use_qk_norm)
+        li = cache.write(k, v)
     special = attn.window or attn.sinks is not None or attn.scale is not None or attn.softcap
     if special and cache.mode == "prefill":
         o = attn.masked_core(q, k, v, ctx)

@@ -175,6 +175,38 @@ def test_decode_attention_parts(B, S, heads, kv_heads, D):
     assert ((got - want)[fine].abs() <= 2.0 ** -8 * want[fine].abs() + 1e-4).all()
 
 
+@pytest.mark.parametrize("T,heads,kv_heads,norm", [(1, 32, 4, True), (5, 3, 1, True), (70, 24, 8, False)])
+def test_rotation_with_cache_write_equals_the_separate_steps(T, heads, kv_heads, norm):
+    """Bit for bit against the rotation kernel followed by the scatter; a position past the cache is dropped and recorded."""
+    from types import SimpleNamespace
+
+    from halo_b200.inference.generate import KVCache
+    from halo_b200.ops import _lib
+    from halo_b200.ops.rope import qk_norm_rope, rope_table
+
+    torch.manual_seed(T)
+    B, S = 3, 40
+    cfg = SimpleNamespace(num_attention_heads=heads, num_key_value_heads=kv_heads, head_dim=128, rms_norm_eps=1e-6, use_qk_norm=norm)
+    w = [(1 + 0.1 * torch.randn(128, device="cuda")).bfloat16() for _ in range(2)]
+    attn = SimpleNamespace(cfg=cfg, q_norm=w[0], k_norm=w[1])
+    qkv = torch.randn(T, (heads + 2 * kv_heads) * 128, device="cuda").bfloat16()
+    places = torch.randperm(B * S, device="cuda")[:T]
+    caches = [KVCache(2, B, S, kv_heads, 128, torch.bfloat16, "cuda") for _ in range(2)]
+    for c in caches:
+        c._rows, c._cols, c._layer = places // S, places % S, 1
+    table = rope_table(caches[0]._cols, 128, 1e6)
+    q, k, li = caches[0].rotate_and_write(qkv, attn, table, keep_keys=True)
+    want_q, want_k = qk_norm_rope(qkv, w[0], w[1], table, heads, kv_heads, 1e-6, norm)
+    assert caches[1].write(want_k, qkv[:, (heads + kv_heads) * 128:]) == li == 1
+    assert torch.equal(q, want_q) and torch.equal(k, want_k)
+    assert torch.equal(caches[0].k, caches[1].k) and torch.equal(caches[0].v, caches[1].v)
+    assert _lib.read_status() == 0
+    caches[0]._cols = torch.full_like(places, S)
+    before, caches[0]._layer = caches[0].k.clone(), 0
+    assert caches[0].rotate_and_write(qkv, attn, table, keep_keys=False)[1] is None
+    assert torch.equal(caches[0].k, before) and _lib.read_status() == 4
+
+
 def test_generation_on_gpu_matches_teacher_forcing():
     """Greedy sampling through the cache (packed prefill on the flash kernel, decode kernel) against the full forward of
     the grown sequence at every step."""
