@@ -77,6 +77,12 @@ class _SwiGLULinear(torch.autograd.Function):
         return dx, dw, None
 
 
+def _swiglu_linear(x, w_gate_up):
+    if x.is_cuda and _lib.plain_inference():
+        return gemm.swiglu_matmul(x, w_gate_up)[0]
+    return _SwiGLULinear.apply(x, w_gate_up, torch.is_grad_enabled())
+
+
 class _RouterLinear(torch.autograd.Function):
     """fp32 router logits from bf16 operands (fp32 accumulate, fp32 result)."""
 
@@ -318,7 +324,7 @@ class DenseMLP(nn.Module):
 
             act = _SwiGLULinear.apply(gather_seq(h, ctx.tp), self.gate_up_proj, torch.is_grad_enabled())
             return row_parallel_linear(act, self.down_proj, ctx.tp)
-        return gemm.linear(_SwiGLULinear.apply(h, self.gate_up_proj, torch.is_grad_enabled()), self.down_proj)
+        return gemm.linear(_swiglu_linear(h, self.gate_up_proj), self.down_proj)
 
 
 class SparseMoE(nn.Module):

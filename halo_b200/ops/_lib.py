@@ -95,7 +95,16 @@ def ptr(t: torch.Tensor | None) -> c_void_p:
 
 
 def stream_ptr(device: torch.device | None = None) -> c_void_p:
-    return c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    """The current stream's handle, read without building a stream object (which costs more than a small kernel's launch)."""
+    index = device.index if device is not None and device.index is not None else torch.cuda.current_device()
+    return c_void_p(torch._C._cuda_getCurrentRawStream(index))
+
+
+def plain_inference() -> bool:
+    """True where an operation may call its kernels without its autograd node: gradients are off and neither forward-mode
+    differentiation nor a functorch transform (vmap, grad, jvp) is active, so the node would record and pass on nothing."""
+    return (not torch.is_grad_enabled() and torch.autograd.forward_ad._current_level < 0
+            and torch._C._functorch.peek_interpreter_stack() is None)
 
 
 def check(rc: int, what: str) -> None:

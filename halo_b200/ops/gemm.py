@@ -174,4 +174,6 @@ class _Linear(torch.autograd.Function):
 def linear(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     """``x @ weight.T`` with all three products on the tcgen05 kernel (no bias: the model families
     built here have none on their projections)."""
+    if _lib.plain_inference():
+        return matmul(x.reshape(-1, x.shape[-1]), weight).reshape(*x.shape[:-1], weight.shape[0])
     return _Linear.apply(x, weight)

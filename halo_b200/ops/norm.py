@@ -11,6 +11,8 @@ halo/model_loading/liger/fused_modules.py:120-123).
 
 from __future__ import annotations
 
+import functools
+
 import torch
 
 from . import _lib
@@ -24,31 +26,37 @@ def rms_norm_reference(x, weight, eps, residual=None):
     return (y, h) if residual is not None else y
 
 
+@functools.lru_cache(maxsize=64)
 def _supported(H: int) -> bool:
     return bool(_lib.lib().halo_rmsnorm_supported(_lib.c_int(H)))
+
+
+def _forward(x, residual, weight, eps, save: bool):
+    """The forward kernel: ``(y, h, rstd)`` as rows, ``h`` the normed input (``x`` itself without a residual)."""
+    H = x.shape[-1]
+    x2 = x.reshape(-1, H).contiguous()
+    r2 = residual.reshape(-1, H).contiguous() if residual is not None else None
+    rows = x2.shape[0]
+    y = torch.empty_like(x2)
+    h = torch.empty_like(x2) if r2 is not None else x2
+    rstd = torch.empty(rows, dtype=torch.float32, device=x.device) if save else None
+    rc = _lib.lib().halo_rmsnorm_fwd(
+        _lib.ptr(x2), _lib.ptr(r2), _lib.ptr(weight), _lib.ptr(y), _lib.ptr(h if r2 is not None else None),
+        _lib.ptr(rstd), _lib.c_ll(rows), _lib.c_int(H), _lib.c_float(eps), _lib.stream_ptr(x.device),
+    )
+    _lib.check(rc, "halo_rmsnorm_fwd")
+    return y, h, rstd
 
 
 class _RMSNorm(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, residual, weight, eps):
         shape = x.shape
-        H = shape[-1]
-        x2 = x.reshape(-1, H).contiguous()
-        r2 = residual.reshape(-1, H).contiguous() if residual is not None else None
-        rows = x2.shape[0]
-        y = torch.empty_like(x2)
-        h = torch.empty_like(x2) if r2 is not None else x2
-        rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
-        L = _lib.lib()
-        rc = L.halo_rmsnorm_fwd(
-            _lib.ptr(x2), _lib.ptr(r2), _lib.ptr(weight), _lib.ptr(y), _lib.ptr(h if r2 is not None else None),
-            _lib.ptr(rstd), _lib.c_ll(rows), _lib.c_int(H), _lib.c_float(eps), _lib.stream_ptr(x.device),
-        )
-        _lib.check(rc, "halo_rmsnorm_fwd")
+        y, h, rstd = _forward(x, residual, weight, eps, True)
         ctx.save_for_backward(h, weight, rstd)
-        ctx.has_res = r2 is not None
+        ctx.has_res = residual is not None
         ctx.shape = shape
-        if r2 is not None:
+        if residual is not None:
             return y.reshape(shape), h.reshape(shape)
         return y.reshape(shape), None
 
@@ -76,6 +84,8 @@ class _RMSNorm(torch.autograd.Function):
 def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6) -> torch.Tensor:
     if not x.is_cuda or x.dtype != torch.bfloat16 or not _supported(x.shape[-1]):
         return rms_norm_reference(x, weight, eps)
+    if _lib.plain_inference():
+        return _forward(x, None, weight, eps, False)[0].reshape(x.shape)
     return _RMSNorm.apply(x, None, weight, eps)[0]
 
 
@@ -83,4 +93,7 @@ def add_rms_norm(x: torch.Tensor, residual: torch.Tensor, weight: torch.Tensor, 
     """Returns ``(rms_norm(x + residual), x + residual)``."""
     if not x.is_cuda or x.dtype != torch.bfloat16 or not _supported(x.shape[-1]):
         return rms_norm_reference(x, weight, eps, residual)
+    if _lib.plain_inference():
+        y, h, _ = _forward(x, residual, weight, eps, False)
+        return y.reshape(x.shape), h.reshape(x.shape)
     return _RMSNorm.apply(x, residual, weight, eps)
