@@ -16,6 +16,8 @@
 // (halo/models/attention/selection.py:94-100, 383-462).
 #include "sm100_common.cuh"
 
+#include <type_traits>
+
 #include <stdio.h>
 #include <stdlib.h>
 
@@ -28,6 +30,15 @@ int make_tmap_bf16(CUtensorMap* m, const void* base, long long rows, long long c
                    int box_rows);  // gemm_sm100.cu
 
 // 2^x on the special-function unit (one MUFU op; inputs here are <= 8 after max subtraction)
+// (x.x * m + a, x.y * m + a) in one packed operation
+__device__ __forceinline__ float2 fma2(float2 x, float m, float a) {
+    float2 r;
+    asm("{\n\t.reg .b64 x, m, a, d;\n\t"
+        "mov.b64 x, {%2, %3};\n\tmov.b64 m, {%4, %4};\n\tmov.b64 a, {%5, %5};\n\t"
+        "fma.rn.f32x2 d, x, m, a;\n\tmov.b64 {%0, %1}, d;\n\t}"
+        : "=f"(r.x), "=f"(r.y) : "f"(x.x), "f"(x.y), "f"(m), "f"(a));
+    return r;
+}
 __device__ __forceinline__ float fast_exp2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -830,18 +841,20 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 // Backward, second form. Same tiling and the same deterministic split into a dK/dV kernel and a dQ kernel as above,
 // rebuilt around the fact that one step is a chain of latencies (products -> TMEM loads -> exp / mask / scale ->
 // shared-memory stores -> products), not of throughput:
-//   * the score / dP accumulators (tensor memory) and the P^T / dS^T operand tiles (shared memory) exist twice, and TWO
-//     groups of eight element-wise warps alternate steps (group g takes the steps with it % 2 == g and always works on
-//     copy g), so two steps' chains are in flight and the products of step i+1 are issued before the element-wise pass
-//     of step i has finished;
-//   * inside a group each thread owns one row and 32 of its 64 columns, so it holds 32 score values, not 64;
-//   * the streamed operand tiles (Q, dO for dK/dV; K, V for dQ) have three / four stages, so that their loads are in
-//     flight two steps ahead and the round trip to L2 never sits between two steps.
+//   * the score / dP accumulators exist twice in tensor memory, so the products of step i + 1 are issued before the
+//     element-wise pass of step i has finished; P^T / dS^T go over the columns their scores came from;
+//   * all sixteen element-wise warps work on every step, a thread on one row and 16 of its 64 columns. The products of step
+//     i + 2 wait for step i's dS, so what counts is how soon a step is done: two groups of eight warps that took alternate
+//     steps had the same throughput and twice the latency (dQ 2,360 us against 1,930 with operands in tensor memory as well,
+//     dK/dV 2,380 against 2,160, for 65,536 tokens of chat documents, 32 / 4 heads);
+//   * the streamed operand tiles (Q, dO for dK/dV; K, V for dQ) have five stages, so that their loads are in
+//     flight ahead and the round trip to L2 never sits between two steps;
+//   * the MMA warp walks its loop as a whole (see elect_one).
 //   warp 0: TMA producer, warp 1: MMA issuer, warps 2..17: element-wise
-//   (group = (warp - 2) / 8, TMEM lane quarter = warp & 3, column half = ((warp - 2) % 8) / 4)
+//   (TMEM lane quarter = warp & 3, column part = (warp - 2) / 4)
 // ---------------------------------------------------------------------------------------------
 constexpr int kBwd2Threads = 576;
-constexpr int kBwd2Ew = 256;                      // element-wise threads of one group
+constexpr int kBwd2Ew = 512;                      // element-wise threads
 constexpr int kBwd2EwWarps = kBwd2Ew / 32;        // a warp arrives on a barrier once, through its first lane
 
 // All lanes of the warp have finished what the barrier publishes (their loads from tensor memory, their stores and
@@ -852,15 +865,16 @@ __device__ __forceinline__ void warp_arrive(uint32_t bar, int lane) {
     if (lane == 0) mbar_arrive(bar);
 }
 
-__device__ __forceinline__ void ew_bar_sync(int group) {   // named barrier of one group's eight warps
-    asm volatile("bar.sync %0, %1;" ::"r"(2 + group), "n"(kBwd2Ew) : "memory");
+__device__ __forceinline__ void ew_bar_sync() {
+    asm volatile("bar.sync 1, %0;" ::"n"(kBwd2Ew) : "memory");
 }
 
 // K, V (32 KiB each), 5 stages of (Q, dO) 64 x 128 (16 KiB each). P^T and dS^T never touch shared memory: every
 // element-wise thread writes its row of them (bf16 pairs) with tcgen05.st over the tensor-memory columns its scores
 // came from, and the dV / dK products take their A operand from there. (Measured per step of this kernel before:
 // the MMA thread spent 2,100 of 3,700 cycles blocked in issue, because operand fetches, the element-wise stores and the
-// TMA writes share one 128-byte-per-clock shared-memory port.)
+// TMA writes share one 128-byte-per-clock shared-memory port.) K and V stay shared-memory operands here - 48 cycles a
+// 128 x 64 x 16 product instead of 32 -: the accumulators fill tensor memory.
 constexpr int kBwdKv2Stages = 5;
 constexpr int kBwdKv2Tiles = 2 * kTileBytes + kBwdKv2Stages * 2 * kHalfTile;     // 229,376
 constexpr int kBwdKv2Smem = kBwdKv2Tiles + 2048;                                                 // barriers, scalars, statistics
@@ -881,8 +895,8 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     enum { kKv = 0, kQFull = 1, kQEmpty = 6, kSFull = 11, kPReady = 13, kDsReady = 15, kAccDone = 17, kNumBars = 18 };
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kNumBars);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + kNumBars + 1);
-    float* s_lse = reinterpret_cast<float*>(bars + kNumBars + 2);          // [2 groups][64]
-    float* s_delta = s_lse + 128;                                          // [2 groups][64]
+    float* s_lse = reinterpret_cast<float*>(bars + kNumBars + 2);          // [2 copies][64]
+    float* s_delta = s_lse + 128;                                          // [2 copies][64]
     auto bar = [&](int i) { return smem_u32(&bars[i]); };
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -914,7 +928,7 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     if (threadIdx.x == 0) {
         *abort_flag = 0;
         for (int i = 0; i < kNumBars; ++i) {
-            const bool many = (i >= kPReady && i < kAccDone);      // arrived on by every warp of one element-wise group
+            const bool many = (i >= kPReady && i < kAccDone);      // arrived on by every element-wise warp
             mbar_init(bar(i), many ? kBwd2EwWarps : 1);
         }
         mbar_fence_init();
@@ -928,8 +942,8 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     tc_fence_after();
     const uint32_t tm0 = *tmem_slot;
     // S^T[b] at 128 b, dP^T[b] at 128 b + 64, dV at 256, dK at 384. P^T[b] is written over S^T[b] and dS^T[b] over
-    // dP^T[b]: the 32 queries of column half h as 16 packed columns at offset 32 h, i.e. inside the columns the writing
-    // thread has itself just read, so the two halves' warps need no order between them.
+    // dP^T[b]: 16 queries as 8 packed columns at their own offset, i.e. inside the columns the writing thread has itself just
+    // read, so the four column parts' warps need no order between them.
     const uint32_t tDV = tm0 + 256, tDK = tm0 + 384;
 
     if (warp == 0) {
@@ -963,70 +977,71 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc_st = make_idesc_bf16(128, 64, 0, 0);   // [keys x q] = K Q^T, V dO^T
-            constexpr uint32_t idesc_acc = make_idesc_bf16(128, 128, 0, 1); // [keys x hd] = P^T dO, dS^T Q
-            bool ok = mbar_wait(bar(kKv), 0, abort_flag, p.status);
-            auto issue_s = [&](int j) -> bool {
-                const int b = j & 1, st = j % kBwdKv2Stages;
-                const uint32_t sQ = sQdO + st * 2 * kHalfTile, sdO = sQ + kHalfTile;
-                if (!mbar_wait(bar(kQFull + st), (j / kBwdKv2Stages) & 1, abort_flag, p.status)) return false;   // Q, dO of step j
-                // S^T / dP^T[b] are free: their last readers are the dV / dK products of step j - 2, which this thread
-                // issued before this point, and the tensor pipe runs one thread's products in order
-                tc_fence_after();
-                const uint32_t tS = tm0 + 128 * b, tDP = tS + 64;
+        // the whole warp walks the loop, one lane issues (see elect_one)
+        constexpr uint32_t idesc_st = make_idesc_bf16(128, 64, 0, 0);   // [keys x q] = K Q^T, V dO^T
+        constexpr uint32_t idesc_acc = make_idesc_bf16(128, 128, 0, 1); // [keys x hd] = P^T dO, dS^T Q
+        const uint64_t desc_k = make_smem_desc(sK, 16, 1024), desc_v = make_smem_desc(sV, 16, 1024);
+        bool ok = mbar_wait_warp(bar(kKv), 0, abort_flag, p.status);
+        auto issue_s = [&](int j) -> bool {
+            const int b = j & 1, st = j % kBwdKv2Stages;
+            if (!mbar_wait_warp(bar(kQFull + st), (j / kBwdKv2Stages) & 1, abort_flag, p.status)) return false;   // Q, dO of step j
+            // S^T / dP^T[b] are free: their last readers are the dV / dK products of step j - 2, which this warp
+            // issued before this point, and the tensor pipe runs one thread's products in order
+            tc_fence_after();
+            const uint64_t desc_q = make_smem_desc(sQdO + st * 2 * kHalfTile, 16, 1024);
+            const uint64_t desc_do = make_smem_desc(sQdO + st * 2 * kHalfTile + kHalfTile, 16, 1024);
+            const uint32_t tS = tm0 + 128 * b, tDP = tS + 64;
+            if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < 8; ++ks) {
-                    const uint32_t offa = (ks >> 2) * 16384 + (ks & 3) * 32;  // K / V: 128-row halves
-                    const uint32_t offb = (ks >> 2) * 8192 + (ks & 3) * 32;   // Q / dO: 64-row halves
-                    tc_mma_f16(tS, make_smem_desc(sK + offa, 16, 1024), make_smem_desc(sQ + offb, 16, 1024), idesc_st, ks != 0);
-                }
+                for (int ks = 0; ks < 8; ++ks)       // K / V: 128-row halves, Q / dO: 64-row halves
+                    tc_mma_f16(tS, desc_k + ((ks >> 2) * 16384 + (ks & 3) * 32) / 16, desc_q + ((ks >> 2) * 8192 + (ks & 3) * 32) / 16,
+                               idesc_st, ks != 0);
 #pragma unroll
-                for (int ks = 0; ks < 8; ++ks) {
-                    const uint32_t offa = (ks >> 2) * 16384 + (ks & 3) * 32;
-                    const uint32_t offb = (ks >> 2) * 8192 + (ks & 3) * 32;
-                    tc_mma_f16(tDP, make_smem_desc(sV + offa, 16, 1024), make_smem_desc(sdO + offb, 16, 1024), idesc_st, ks != 0);
-                }
+                for (int ks = 0; ks < 8; ++ks)
+                    tc_mma_f16(tDP, desc_v + ((ks >> 2) * 16384 + (ks & 3) * 32) / 16,
+                               desc_do + ((ks >> 2) * 8192 + (ks & 3) * 32) / 16, idesc_st, ks != 0);
                 tc_commit(bar(kSFull + b));
-                return true;
-            };
-            if (ok && n_iter > 0) ok = issue_s(0);
-            for (int it = 0; ok && it < n_iter; ++it) {
-                const int b = it & 1, st = it % kBwdKv2Stages;
-                const uint32_t sQ = sQdO + st * 2 * kHalfTile, sdO = sQ + kHalfTile;
-                if (it + 1 < n_iter && !issue_s(it + 1)) break;
-                if (!mbar_wait(bar(kPReady + b), (it >> 1) & 1, abort_flag, p.status)) break;      // P^T[b] written
-                tc_fence_after();
-                const uint32_t tPT = tm0 + 128 * b, tDST = tPT + 64;
-#pragma unroll
-                for (int ks = 0; ks < 4; ++ks)   // 16 queries = 8 packed columns per step; queries 32.. sit at column 32
-                    tc_mma_f16_tmem_a(tDV, tPT + (ks >> 1) * 32 + (ks & 1) * 8,
-                                      make_smem_desc(sdO + ks * 2048, 8192, 1024), idesc_acc, (it | ks) != 0);
-                if (!mbar_wait(bar(kDsReady + b), (it >> 1) & 1, abort_flag, p.status)) break;     // dS^T[b] written
-                tc_fence_after();
+            }
+            __syncwarp();
+            return true;
+        };
+        if (ok && n_iter > 0) ok = issue_s(0);
+        for (int it = 0; ok && it < n_iter; ++it) {
+            const int b = it & 1, st = it % kBwdKv2Stages;
+            if (it + 1 < n_iter && !issue_s(it + 1)) break;
+            const uint64_t desc_qt = make_smem_desc(sQdO + st * 2 * kHalfTile, 8192, 1024);
+            const uint64_t desc_dot = make_smem_desc(sQdO + st * 2 * kHalfTile + kHalfTile, 8192, 1024);
+            const uint32_t tPT = tm0 + 128 * b, tDST = tPT + 64;       // 16 queries = 8 packed columns per step, 16 apart
+            if (!mbar_wait_warp(bar(kPReady + b), (it >> 1) & 1, abort_flag, p.status)) break;      // P^T[b] written
+            tc_fence_after();
+            if (elect_one()) {
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks)
-                    tc_mma_f16_tmem_a(tDK, tDST + (ks >> 1) * 32 + (ks & 1) * 8,
-                                      make_smem_desc(sQ + ks * 2048, 8192, 1024), idesc_acc, (it | ks) != 0);
+                    tc_mma_f16_tmem_a(tDV, tPT + ks * 16, desc_dot + ks * 2048 / 16, idesc_acc, (it | ks) != 0);
+            }
+            __syncwarp();
+            if (!mbar_wait_warp(bar(kDsReady + b), (it >> 1) & 1, abort_flag, p.status)) break;     // dS^T[b] written
+            tc_fence_after();
+            if (elect_one()) {
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks)
+                    tc_mma_f16_tmem_a(tDK, tDST + ks * 16, desc_qt + ks * 2048 / 16, idesc_acc, (it | ks) != 0);
                 tc_commit(bar(kQEmpty + st));
                 if (it == n_iter - 1) tc_commit(bar(kAccDone));
             }
+            __syncwarp();
         }
     } else {
-        const int g = (warp - 2) >> 3;                            // element-wise group: steps with it % 2 == g, copy g of everything
-        const int quad = warp & 3, half = ((warp - 2) & 7) >> 2;
-        const int ew_tid = (threadIdx.x - 64) & (kBwd2Ew - 1);    // index inside the group
+        // all sixteen warps work on every step, sixteen queries of it each
+        const int quad = warp & 3, part = (warp - 2) >> 2;
+        const int ew_tid = threadIdx.x - 64;
         const int key = quad * 32 + lane;                         // this thread's key row of the tile
-        const int c0 = half * 32;                                 // its first query column
+        const int c0 = part * 16;                                 // its first query column
         const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
         const float c = p.scale * kLog2e;
         const long long key_abs = (long long)w.kv0 + key;
-        const uint32_t tS = tm0 + 128 * g + lane_base + c0, tDP = tS + 64;
-        const uint32_t tPT = tm0 + 128 * g + lane_base + c0, tDST = tPT + 64;   // this thread's 16 packed columns of P^T / dS^T
-        float* lse_g = s_lse + g * 64;
-        float* delta_g = s_delta + g * 64;
         bool ok = true;
-        // statistics of a step, fetched by the group's first 128 threads (64 lse, 64 delta) one of its steps ahead
+        // statistics of a step (64 lse, 64 delta): fetched by the first 128 threads two steps ahead, put down one step ahead
         auto fetch_stat = [&](int it) -> float {
             if (ew_tid >= 128 || it >= n_iter) return 0.f;
             const int h = kv_head * group + it % group;
@@ -1036,23 +1051,30 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             if (ew_tid < 64) return in ? p.lse[(long long)h * p.T + ql] * kLog2e : INFINITY;
             return in ? p.delta[(long long)h * p.T + ql] : 0.f;
         };
-        float stat = fetch_stat(g);
-        for (int it = g; it < n_iter; it += 2) {
-            const int k = it >> 1;                                // this group's step count: parity of its barriers
+        auto put_stat = [&](int it, float v) {
+            if (ew_tid < 64) s_lse[(it & 1) * 64 + ew_tid] = v;
+            else if (ew_tid < 128) s_delta[(it & 1) * 64 + ew_tid - 64] = v;
+        };
+        put_stat(0, fetch_stat(0));
+        float stat = fetch_stat(1);
+        for (int it = 0; it < n_iter; ++it) {
+            const int b = it & 1;
             const int qr = q_row(it / group);
-            // Every thread of the group meets at the two barriers below in every one of its steps, also after a wait has
-            // given up (it then skips the step's work): nobody may leave the loop early and strand the others.
-            ew_bar_sync(g);                                       // the previous step's readers of the statistics are done
-            if (ew_tid < 64) lse_g[ew_tid] = stat;
-            else if (ew_tid < 128) delta_g[ew_tid - 64] = stat;
-            stat = fetch_stat(it + 2);                            // in flight during this step
-            ew_bar_sync(g);
+            const uint32_t tS = tm0 + 128 * b + lane_base + c0, tDP = tS + 64;
+            // Every thread meets at the barrier below in every step, also after a wait has given up (it then skips the step's
+            // work): nobody may leave the loop early and strand the others. Behind it this step's statistics are in place and
+            // the previous step's have been read.
+            ew_bar_sync();
+            put_stat(it + 1, stat);
+            stat = fetch_stat(it + 2);
             if (!ok) continue;
-            if (!mbar_wait(bar(kSFull + g), k & 1, abort_flag, p.status)) { ok = false; continue; }
+            const float* lse_b = s_lse + b * 64 + c0;
+            const float* delta_b = s_delta + b * 64 + c0;
+            if (!mbar_wait(bar(kSFull + b), (it >> 1) & 1, abort_flag, p.status)) { ok = false; continue; }
             tc_fence_after();
-            uint32_t sr[32], dr[32];
-            tmem_ld_32x32(tS, sr);
-            tmem_ld_32x32(tDP, dr);
+            uint32_t sr[16], dr[16];
+            tmem_ld_32x16(tS, sr);
+            tmem_ld_32x16(tDP, dr);
             tmem_ld_wait();
             // Only the tiles on the diagonal need the causal mask; everywhere else the loop carries no compare at all.
             // Column i of this thread is query qr + c0 + i; it sees key `key_abs` when i >= lim.
@@ -1060,41 +1082,32 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             const bool need_mask = (qr < w.kv0 + 128) || (kWin && qr + 63 - w.kv0 >= p.window);
             const int lim = (int)(key_abs - qr) - c0;
             const int hi = kWin ? lim + p.window : 0;
-            float pv[32];
+            float pv[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) pv[i] = fast_exp2(__uint_as_float(sr[i]) * c - lse_b[i]);
             if (need_mask) {
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    const float pe = fast_exp2(__uint_as_float(sr[i]) * c - lse_g[c0 + i]);
-                    pv[i] = (i < lim || (kWin && i >= hi)) ? 0.f : pe;
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) pv[i] = fast_exp2(__uint_as_float(sr[i]) * c - lse_g[c0 + i]);
+                for (int i = 0; i < 16; ++i) pv[i] = (i < lim || (kWin && i >= hi)) ? 0.f : pv[i];
             }
-            // P^T[g]: this thread's 32 probabilities as 16 packed columns, over the score columns it has just read
-            {
-                uint32_t pk[16];
+            uint32_t pk[8];
 #pragma unroll
-                for (int i = 0; i < 16; ++i) pk[i] = pack_bf16(pv[2 * i], pv[2 * i + 1]);
-                tmem_st_32x16(tPT, pk);
-                tmem_st_wait();
-            }
+            for (int i = 0; i < 8; ++i) pk[i] = pack_bf16(pv[2 * i], pv[2 * i + 1]);
+            tmem_st_32x8(tS, pk);                                 // P^T: over the score columns this thread has just read
+            tmem_st_wait();
             tc_fence_before();
-            warp_arrive(bar(kPReady + g), lane);
+            warp_arrive(bar(kPReady + b), lane);
             // dS^T = P^T * (dP^T - delta) * scale
 #pragma unroll
-            for (int i = 0; i < 32; ++i) pv[i] = pv[i] * (__uint_as_float(dr[i]) - delta_g[c0 + i]) * p.scale;
-            {
-                uint32_t pk[16];
+            for (int i = 0; i < 16; ++i) pv[i] = pv[i] * (__uint_as_float(dr[i]) - delta_b[i]) * p.scale;
 #pragma unroll
-                for (int i = 0; i < 16; ++i) pk[i] = pack_bf16(pv[2 * i], pv[2 * i + 1]);
-                tmem_st_32x16(tDST, pk);
-                tmem_st_wait();
-            }
+            for (int i = 0; i < 8; ++i) pk[i] = pack_bf16(pv[2 * i], pv[2 * i + 1]);
+            tmem_st_32x8(tDP, pk);
+            tmem_st_wait();
             tc_fence_before();
-            warp_arrive(bar(kDsReady + g), lane);
+            warp_arrive(bar(kDsReady + b), lane);
         }
-        // the accumulators: group 0 stores dK, group 1 stores dV (each thread one row, 64 of its 128 columns)
+        // the accumulators: parts 0 and 1 store dK, 2 and 3 dV (each thread one row, 64 of its 128 columns)
+        const int g = part >> 1, half = part & 1;
         if (ok && mbar_wait(bar(kAccDone), 0, abort_flag, p.status)) {
             tc_fence_after();
             bool live = key_abs < w.q_end;
@@ -1166,7 +1179,7 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         return;
     }
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem_q2 + kBwdQ2Tiles);
-    enum { kQ = 0, kKvFull = 1, kKvEmpty = 6, kSFull = 11, kDsReady = 13, kAccDone = 15, kNumBars = 16 };
+    enum { kQ = 0, kKvFull = 1, kKvEmpty = 6, kSFull = 11, kDsReady = 13, kAccDone = 15, kOperands = 16, kNumBars = 17 };
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kNumBars);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + kNumBars + 1);
     auto bar = [&](int i) { return smem_u32(&bars[i]); };
@@ -1184,7 +1197,8 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
     if (threadIdx.x == 0) {
         *abort_flag = 0;
-        for (int i = 0; i < kNumBars; ++i) mbar_init(bar(i), (i >= kDsReady && i < kAccDone) ? kBwd2EwWarps : 1);
+        for (int i = 0; i < kNumBars; ++i)          // the element-wise warps arrive once each
+            mbar_init(bar(i), (i == kOperands || (i >= kDsReady && i < kAccDone)) ? kBwd2EwWarps : 1);
         mbar_fence_init();
     }
     if (warp == 1) {
@@ -1196,6 +1210,9 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     tc_fence_after();
     const uint32_t tm0 = *tmem_slot;
     const uint32_t tDQ = tm0 + 256;     // S[b] at 128 b, dP[b] at 128 b + 64
+    // Q and dO as packed bf16 pairs, 64 columns each: the A operands of every step. A 128 x 64 x 16 product that reads them from
+    // shared memory takes 48 cycles, bound by the port; from tensor memory 32.
+    const uint32_t tQ = tm0 + 384, tdO = tm0 + 448;
 
     if (warp == 0) {
         if (lane == 0) {
@@ -1227,52 +1244,51 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc_s = make_idesc_bf16(128, 64, 0, 0);     // [q x keys]
-            constexpr uint32_t idesc_dq = make_idesc_bf16(128, 128, 0, 1);   // [q x hd] = dS K
-            bool ok = mbar_wait(bar(kQ), 0, abort_flag, p.status);
-            auto issue_s = [&](int j) -> bool {
-                const int b = j & 1, st = j % kBwdQ2Stages;
-                const uint32_t sK = sKV + st * 2 * kHalfTile, sV = sK + kHalfTile;
-                if (!mbar_wait(bar(kKvFull + st), (j / kBwdQ2Stages) & 1, abort_flag, p.status)) return false;
-                tc_fence_after();       // S / dP[b]: last read by the dQ product of step j - 2, issued before this point
-                const uint32_t tS = tm0 + 128 * b, tDP = tS + 64;
+        // the whole warp walks the loop, one lane issues (see elect_one)
+        constexpr uint32_t idesc_s = make_idesc_bf16(128, 64, 0, 0);     // [q x keys]
+        constexpr uint32_t idesc_dq = make_idesc_bf16(128, 128, 0, 1);   // [q x hd] = dS K
+        bool ok = mbar_wait_warp(bar(kOperands), 0, abort_flag, p.status);
+        auto issue_s = [&](int j) -> bool {
+            const int b = j & 1, st = j % kBwdQ2Stages;
+            if (!mbar_wait_warp(bar(kKvFull + st), (j / kBwdQ2Stages) & 1, abort_flag, p.status)) return false;
+            tc_fence_after();       // S / dP[b]: last read by the dQ product of step j - 2, issued before this point
+            const uint64_t desc_k = make_smem_desc(sKV + st * 2 * kHalfTile, 16, 1024);
+            const uint64_t desc_v = make_smem_desc(sKV + st * 2 * kHalfTile + kHalfTile, 16, 1024);
+            const uint32_t tS = tm0 + 128 * b, tDP = tS + 64;
+            if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < 8; ++ks) {
-                    const uint32_t offa = (ks >> 2) * 16384 + (ks & 3) * 32;
-                    const uint32_t offb = (ks >> 2) * 8192 + (ks & 3) * 32;
-                    tc_mma_f16(tS, make_smem_desc(sQ + offa, 16, 1024), make_smem_desc(sK + offb, 16, 1024), idesc_s, ks != 0);
-                }
+                for (int ks = 0; ks < 8; ++ks)
+                    tc_mma_f16_tmem_a(tS, tQ + ks * 8, desc_k + ((ks >> 2) * 8192 + (ks & 3) * 32) / 16, idesc_s, ks != 0);
 #pragma unroll
-                for (int ks = 0; ks < 8; ++ks) {
-                    const uint32_t offa = (ks >> 2) * 16384 + (ks & 3) * 32;
-                    const uint32_t offb = (ks >> 2) * 8192 + (ks & 3) * 32;
-                    tc_mma_f16(tDP, make_smem_desc(sdO + offa, 16, 1024), make_smem_desc(sV + offb, 16, 1024), idesc_s, ks != 0);
-                }
+                for (int ks = 0; ks < 8; ++ks)
+                    tc_mma_f16_tmem_a(tDP, tdO + ks * 8, desc_v + ((ks >> 2) * 8192 + (ks & 3) * 32) / 16, idesc_s, ks != 0);
                 tc_commit(bar(kSFull + b));
-                return true;
-            };
-            if (ok && w.n_kv > 0) ok = issue_s(0);
-            for (int j = 0; ok && j < w.n_kv; ++j) {
-                const int b = j & 1, st = j % kBwdQ2Stages;
-                const uint32_t sK = sKV + st * 2 * kHalfTile;
-                if (j + 1 < w.n_kv && !issue_s(j + 1)) break;
-                if (!mbar_wait(bar(kDsReady + b), (j >> 1) & 1, abort_flag, p.status)) break;
-                tc_fence_after();
-                const uint32_t tDS = tm0 + 128 * b + 64;      // dS[b], written over dP[b]
+            }
+            __syncwarp();
+            return true;
+        };
+        if (ok && w.n_kv > 0) ok = issue_s(0);
+        for (int j = 0; ok && j < w.n_kv; ++j) {
+            const int b = j & 1, st = j % kBwdQ2Stages;
+            if (j + 1 < w.n_kv && !issue_s(j + 1)) break;
+            if (!mbar_wait_warp(bar(kDsReady + b), (j >> 1) & 1, abort_flag, p.status)) break;
+            tc_fence_after();
+            const uint32_t tDS = tm0 + 128 * b + 64;      // dS[b], written over dP[b]: 16 keys as 8 packed columns, 16 apart
+            const uint64_t desc_kt = make_smem_desc(sKV + st * 2 * kHalfTile, 8192, 1024);
+            if (elect_one()) {
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks)
-                    tc_mma_f16_tmem_a(tDQ, tDS + (ks >> 1) * 32 + (ks & 1) * 8,
-                                      make_smem_desc(sK + ks * 2048, 8192, 1024), idesc_dq, (j | ks) != 0);
+                    tc_mma_f16_tmem_a(tDQ, tDS + ks * 16, desc_kt + ks * 2048 / 16, idesc_dq, (j | ks) != 0);
                 tc_commit(bar(kKvEmpty + st));
                 if (j == w.n_kv - 1) tc_commit(bar(kAccDone));
             }
+            __syncwarp();
         }
     } else {
-        const int g = (warp - 2) >> 3;
-        const int quad = warp & 3, half = ((warp - 2) & 7) >> 2;
+        // all sixteen warps work on every step, sixteen keys of it each
+        const int quad = warp & 3, part = (warp - 2) >> 2;
         const int row = quad * 32 + lane;
-        const int c0 = half * 32;
+        const int c0 = part * 16;
         const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
         const float c = p.scale * kLog2e;
         const long long q_abs = (long long)w.q0 + row;
@@ -1280,47 +1296,57 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const long long q_local = q_abs - q_shift;
         const float lse2 = in ? p.lse[(long long)head * p.T + q_local] * kLog2e : INFINITY;
         const float dl = in ? p.delta[(long long)head * p.T + q_local] : 0.f;
-        const uint32_t tS = tm0 + 128 * g + lane_base + c0, tDP = tS + 64;
-        bool ok = true;
-        for (int j = g; j < w.n_kv; j += 2) {
-            const int k = j >> 1;
-            if (!mbar_wait(bar(kSFull + g), k & 1, abort_flag, p.status)) { ok = false; break; }
+        // parts 0 and 1 move Q to tensor memory, 2 and 3 dO: a thread 64 columns (128 swizzled bytes) of its row
+        bool ok = mbar_wait(bar(kQ), 0, abort_flag, p.status);
+        if (ok) {
+            uint32_t a[32];
+            const uint32_t src = (part < 2 ? sQ : sdO) + (part & 1) * 16384 + row * 128;
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(a[4 * u]), "=r"(a[4 * u + 1]), "=r"(a[4 * u + 2]), "=r"(a[4 * u + 3])
+                             : "r"(src + ((u ^ (row & 7)) << 4)));
+            tmem_st_32x32((part < 2 ? tQ : tdO) + lane_base + (part & 1) * 32, a);
+            tmem_st_wait();
+            tc_fence_before();
+            warp_arrive(bar(kOperands), lane);
+        }
+        for (int j = 0; ok && j < w.n_kv; ++j) {
+            const int b = j & 1;
+            const uint32_t tS = tm0 + 128 * b + lane_base + c0, tDP = tS + 64;
+            if (!mbar_wait(bar(kSFull + b), (j >> 1) & 1, abort_flag, p.status)) { ok = false; break; }
             tc_fence_after();
-            uint32_t sr[32], dr[32];
-            tmem_ld_32x32(tS, sr);
-            tmem_ld_32x32(tDP, dr);
+            uint32_t sr[16], dr[16];
+            tmem_ld_32x16(tS, sr);
+            tmem_ld_32x16(tDP, dr);
             tmem_ld_wait();
             // column i of this thread is key k0 + i; the row sees it when i <= lim. Off the diagonal no compare is made.
             const int k0 = w.kv0 + j * 64 + c0;
-            const bool need_mask = (k0 + 32 > w.q0) || (kWin && k0 + p.window <= w.q0 + 127);
+            const bool need_mask = (k0 + 16 > w.q0) || (kWin && k0 + p.window <= w.q0 + 127);
             const int lim = (int)(q_abs - k0);
             const int lo = kWin ? lim - p.window + 1 : 0;                         // first visible column under a window
-            float pv[32];
+            float pv[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                pv[i] = fast_exp2(__uint_as_float(sr[i]) * c - lse2) * (__uint_as_float(dr[i]) - dl) * p.scale;
             if (need_mask) {
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    const float pe = fast_exp2(__uint_as_float(sr[i]) * c - lse2);
-                    pv[i] = (i > lim || (kWin && i < lo)) ? 0.f : pe * (__uint_as_float(dr[i]) - dl) * p.scale;
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < 32; ++i)
-                    pv[i] = fast_exp2(__uint_as_float(sr[i]) * c - lse2) * (__uint_as_float(dr[i]) - dl) * p.scale;
+                for (int i = 0; i < 16; ++i) pv[i] = (i > lim || (kWin && i < lo)) ? 0.f : pv[i];
             }
             {
-                uint32_t pk[16];
+                uint32_t pk[8];
 #pragma unroll
-                for (int i = 0; i < 16; ++i) pk[i] = pack_bf16(pv[2 * i], pv[2 * i + 1]);
-                tmem_st_32x16(tDP, pk);         // this thread's 16 packed columns of dS[g], over the dP columns it has just read
+                for (int i = 0; i < 8; ++i) pk[i] = pack_bf16(pv[2 * i], pv[2 * i + 1]);
+                tmem_st_32x8(tDP, pk);          // this thread's 8 packed columns of dS, over the dP columns it has just read
                 tmem_st_wait();
             }
             tc_fence_before();
-            warp_arrive(bar(kDsReady + g), lane);
+            warp_arrive(bar(kDsReady + b), lane);
         }
-        // the accumulator: every thread of group g stores 32 columns of its row (group, half -> which 32 of the 128)
+        // the accumulator: every thread stores 32 of its row's 128 columns
         if (ok && mbar_wait(bar(kAccDone), 0, abort_flag, p.status)) {
             tc_fence_after();
-            const int col = g * 64 + half * 32;
+            const int col = part * 32;
             __nv_bfloat16* dq = reinterpret_cast<__nv_bfloat16*>(p.dQ) + q_local * p.ld_dq + head * kHd + col;
             uint32_t r[32];
             tmem_ld_32x32(tDQ + lane_base + col, r);
@@ -1362,6 +1388,9 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 // of the stage is dead, so P (same 16 KiB) is written over it and the stage is released after P V.
 constexpr int kFwd2Tiles = kTileBytes + 2 * 2 * kHalfTile;
 constexpr int kFwd2Smem = kFwd2Tiles + 256;                              // + barriers and scalars
+constexpr int kFwd3KeyBuffers = 3;
+constexpr int kFwd3Tiles = kTileBytes + (kFwd3KeyBuffers + 2) * kHalfTile;   // 114,688
+constexpr int kFwd3Smem = kFwd3Tiles + 256;
 
 // 160 registers: six warps of 160 x 32 registers fit twice into the 64K-register file (the
 // allocation granularity makes 168 miss it)
@@ -1607,25 +1636,33 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 // takes its A operand from tensor memory. Shared memory then carries only Q, K and V: a third less traffic per step on
 // the resource that limits this kernel (operand fetches of the products and the K/V loads share one 128-byte-per-clock
 // port), and the proxy fence between the softmax's stores and the product disappears.
+// What bounds it is a tile's chain of latencies: scores, softmax, product, and the loads behind them. Three things shorten it.
+// Keys and values have buffers of their own, so that a key tile's successor is on its way when its scores are formed (24,531
+// tokens of 256-16,384-token documents, 32 / 4 heads: 1,083 -> 851 us; a third key buffer 840 us); a thread reads its 64
+// scores once and takes maximum and sum in four chains each (1,121 -> 1,083 us); and the completion of the previous product
+// is waited for behind the exponentials unless the output has to be rescaled.
 template <bool kCP, bool kWin = false>
-__global__ void __maxnreg__(128)
+__global__ void __maxnreg__(168)
 attn_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const AttnParams p, const __grid_constant__ CpArgs<kCP> ca) {
     if (status_poisoned(p.status)) return;
     extern __shared__ __align__(1024) uint8_t smem3[];
     const uint32_t base = smem_u32(smem3);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem3 + kFwd2Tiles);
-    // bars[0]=q, [1..2]=kv_full, [3..4]=kv_empty, [5]=s_full[0], [6]=p_ready, [7]=o_full, [8]=s_full[1]
-    uint32_t* tmem_slot_p = reinterpret_cast<uint32_t*>(smem3 + kFwd2Tiles + 80);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem3 + kFwd2Tiles + 88);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem3 + kFwd3Tiles);
+    // A key tile's buffer is free as soon as its scores are formed, a softmax and a product before the value tile's; three key
+    // and two value buffers are what two CTAs an SM leave room for.
+    enum { kQ = 0, kKFull = 1, kKEmpty = 4, kVFull = 7, kVEmpty = 9, kSFull = 11, kPReady = 13, kOFull = 14, kNumBars = 15 };
+    uint32_t* tmem_slot_p = reinterpret_cast<uint32_t*>(bars + kNumBars);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + kNumBars + 1);
+    auto bar = [&](int n) { return smem_u32(&bars[n]); };
     if (base & 1023u) {
         if (threadIdx.x == 0 && p.status) atomicCAS(p.status, kStatusOk, kStatusBadArgument);
         return;
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t sQ = base, sKV = base + kTileBytes;
-    const uint32_t bar_q = smem_u32(&bars[0]), bar_p_ready = smem_u32(&bars[6]), bar_o_full = smem_u32(&bars[7]);
-    const uint32_t bar_s_full[2] = {smem_u32(&bars[5]), smem_u32(&bars[8])};
+    const uint32_t sQ = base, sK0 = base + kTileBytes, sV0 = sK0 + kFwd3KeyBuffers * kHalfTile;
+    const uint32_t bar_q = bar(kQ), bar_p_ready = bar(kPReady), bar_o_full = bar(kOFull);
+    const uint32_t bar_s_full[2] = {bar(kSFull), bar(kSFull + 1)};
     const int head = blockIdx.x;
     const int kv_head = head / (p.Hq / p.Hkv);
     const FwdWork w = p.work[blockIdx.y];
@@ -1637,15 +1674,7 @@ attn_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
     if (threadIdx.x == 0) {
         *abort_flag = 0;
-        mbar_init(bar_q, 1);
-        for (int s = 0; s < 2; ++s) {
-            mbar_init(smem_u32(&bars[1 + s]), 1);
-            mbar_init(smem_u32(&bars[3 + s]), 1);
-        }
-        mbar_init(bar_s_full[0], 1);
-        mbar_init(bar_s_full[1], 1);
-        mbar_init(bar_p_ready, 4);            // one arrival per softmax warp
-        mbar_init(bar_o_full, 1);
+        for (int n = 0; n < kNumBars; ++n) mbar_init(bar(n), n == kPReady ? 4 : 1);     // p_ready: one arrival per softmax warp
         mbar_fence_init();
     }
     if (warp == 5) {
@@ -1664,62 +1693,66 @@ attn_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             mbar_expect_tx(bar_q, kTileBytes);
             tma_load_2d(sQ, &tmQ, bar_q, head * kHd, w.q0 - q_shift);
             tma_load_2d(sQ + 16384, &tmQ, bar_q, head * kHd + 64, w.q0 - q_shift);
-            for (int j = 0; j < w.n_kv; ++j) {
-                const int st = j & 1;
-                if (!mbar_wait(smem_u32(&bars[3 + st]), ((j >> 1) & 1) ^ 1u, abort_flag, p.status)) break;
-                const uint32_t full = smem_u32(&bars[1 + st]);
-                const uint32_t sK = sKV + st * 2 * kHalfTile, sV = sK + kHalfTile;
+            auto load = [&](int j, bool value) -> bool {
+                const int depth = value ? 2 : kFwd3KeyBuffers, st = j % depth;
+                if (!mbar_wait(bar((value ? kVEmpty : kKEmpty) + st), ((j / depth) & 1) ^ 1u, abort_flag, p.status)) return false;
+                const uint32_t full = bar((value ? kVFull : kKFull) + st);
+                const uint32_t dst = (value ? sV0 : sK0) + st * kHalfTile;
                 int kr = w.kv0 + j * 64;
-                const CUtensorMap* mapK = &tmK;
-                const CUtensorMap* mapV = &tmV;
+                const CUtensorMap* map = value ? &tmV : &tmK;
                 if constexpr (kCP) {                       // the tile's owner and its row in that rank's published buffer
                     const int pk = cp_piece(ca.cpk, kr);
-                    mapK = &ca.peers.k[ca.cpk.owner[pk]];
-                    mapV = &ca.peers.v[ca.cpk.owner[pk]];
+                    map = value ? &ca.peers.v[ca.cpk.owner[pk]] : &ca.peers.k[ca.cpk.owner[pk]];
                     kr = kr - ca.cpk.bound[pk] + ca.cpk.loc[pk];
                 }
-                mbar_expect_tx(full, 2 * kHalfTile);
-                tma_load_2d(sK, mapK, full, kv_head * kHd, kr);
-                tma_load_2d(sK + 8192, mapK, full, kv_head * kHd + 64, kr);
-                tma_load_2d(sV, mapV, full, kv_head * kHd, kr);
-                tma_load_2d(sV + 8192, mapV, full, kv_head * kHd + 64, kr);
-            }
-        }
-    } else if (warp == 5) {
-        if (lane == 0) {
-            constexpr uint32_t idesc_s = make_idesc_bf16(128, 64, 0, 0);
-            constexpr uint32_t idesc_o = make_idesc_bf16(128, 128, 0, 1);
-            bool ok = mbar_wait(bar_q, 0, abort_flag, p.status);
-            auto issue_s = [&](int j) -> bool {
-                const int st = j & 1;
-                const uint32_t sK = sKV + st * 2 * kHalfTile;
-                if (!mbar_wait(smem_u32(&bars[1 + st]), (j >> 1) & 1, abort_flag, p.status)) return false;
-                tc_fence_after();
-#pragma unroll
-                for (int ks = 0; ks < 8; ++ks) {
-                    const uint32_t offa = (ks >> 2) * 16384 + (ks & 3) * 32;
-                    const uint32_t offb = (ks >> 2) * 8192 + (ks & 3) * 32;
-                    tc_mma_f16(tS + st * 64, make_smem_desc(sQ + offa, 16, 1024),
-                               make_smem_desc(sK + offb, 16, 1024), idesc_s, ks != 0);
-                }
-                tc_commit(bar_s_full[st]);
+                mbar_expect_tx(full, kHalfTile);
+                tma_load_2d(dst, map, full, kv_head * kHd, kr);
+                tma_load_2d(dst + 8192, map, full, kv_head * kHd + 64, kr);
                 return true;
             };
-            if (ok && w.n_kv > 0) ok = issue_s(0);
-            for (int j = 0; ok && j < w.n_kv; ++j) {
-                const int st = j & 1;
-                const uint32_t sK = sKV + st * 2 * kHalfTile, sV = sK + kHalfTile;
-                if (j + 1 < w.n_kv && !issue_s(j + 1)) break;
-                if (!mbar_wait(bar_p_ready, j & 1, abort_flag, p.status)) break;
-                tc_fence_after();
+            // key tiles run two ahead of the value tiles: in the order in which their buffers are freed
+            bool ok = w.n_kv > 0 && load(0, false) && (w.n_kv == 1 || load(1, false));
+            for (int j = 0; ok && j < w.n_kv; ++j)
+                ok = (j + 2 >= w.n_kv || load(j + 2, false)) && load(j, true);
+        }
+    } else if (warp == 5) {
+        // the whole warp walks the loop, one lane issues (see elect_one)
+        constexpr uint32_t idesc_s = make_idesc_bf16(128, 64, 0, 0);
+        constexpr uint32_t idesc_o = make_idesc_bf16(128, 128, 0, 1);
+        const uint64_t desc_q = make_smem_desc(sQ, 16, 1024);
+        bool ok = mbar_wait_warp(bar_q, 0, abort_flag, p.status);
+        auto issue_s = [&](int j) -> bool {
+            const int st = j % kFwd3KeyBuffers;
+            if (!mbar_wait_warp(bar(kKFull + st), (j / kFwd3KeyBuffers) & 1, abort_flag, p.status)) return false;
+            tc_fence_after();
+            const uint64_t desc_k = make_smem_desc(sK0 + st * kHalfTile, 16, 1024);
+            if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < 4; ++ks) {
-                    // P: 16 keys = 8 packed columns per step, in the score buffer of this step
-                    tc_mma_f16_tmem_a(tO, tS + st * 64 + ks * 8, make_smem_desc(sV + ks * 2048, 8192, 1024), idesc_o, (j | ks) != 0);
-                }
-                tc_commit(bar_o_full);
-                tc_commit(smem_u32(&bars[3 + st]));
+                for (int ks = 0; ks < 8; ++ks)      // 16 columns = 32 bytes a step; 64 columns a half
+                    tc_mma_f16(tS + (j & 1) * 64, desc_q + ((ks >> 2) * 16384 + (ks & 3) * 32) / 16,
+                               desc_k + ((ks >> 2) * 8192 + (ks & 3) * 32) / 16, idesc_s, ks != 0);
+                tc_commit(bar_s_full[j & 1]);
+                tc_commit(bar(kKEmpty + st));
             }
+            __syncwarp();
+            return true;
+        };
+        if (ok && w.n_kv > 0) ok = issue_s(0);
+        for (int j = 0; ok && j < w.n_kv; ++j) {
+            const int st = j & 1;
+            if (j + 1 < w.n_kv && !issue_s(j + 1)) break;
+            if (!mbar_wait_warp(bar(kVFull + st), (j >> 1) & 1, abort_flag, p.status)) break;
+            if (!mbar_wait_warp(bar_p_ready, j & 1, abort_flag, p.status)) break;
+            tc_fence_after();
+            const uint64_t desc_v = make_smem_desc(sV0 + st * kHalfTile, 8192, 1024);
+            if (elect_one()) {
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks)      // P: 16 keys = 8 packed columns per step, in the score buffer of this tile
+                    tc_mma_f16_tmem_a(tO, tS + st * 64 + ks * 8, desc_v + ks * 2048 / 16, idesc_o, (j | ks) != 0);
+                tc_commit(bar_o_full);
+                tc_commit(bar(kVEmpty + st));
+            }
+            __syncwarp();
         }
     } else {
         const int row = warp * 32 + lane;
@@ -1738,38 +1771,47 @@ attn_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             const bool need_mask = (k0 + 63 > w.q0) || (kWin && k0 + p.window <= w.q0 + 127);
             const int lim = (int)(q_abs - k0);
             const int lo = kWin ? lim - p.window + 1 : 0;
-            float mx = m_ref;
-#pragma unroll 1
-            for (int half = 0; half < 2; ++half) {
-                uint32_t r[32];
-                tmem_ld_32x32(tSj + lane_base + half * 32, r);
-                tmem_ld_wait();
-                if (need_mask) {
+            // the row's 64 scores, read once; the maximum and the sum run in four chains each, for one chain of 64 dependent
+            // operations would cost more than the exponentials
+            uint32_t r[2][32];
+            tmem_ld_32x32(tSj + lane_base, r[0]);
+            tmem_ld_32x32(tSj + lane_base + 32, r[1]);
+            tmem_ld_wait();
+            if (need_mask) {
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
                     const int lh = lim - half * 32, ll = lo - half * 32;
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) mx = fmaxf(mx, (i <= lh && (!kWin || i >= ll)) ? __uint_as_float(r[i]) : -INFINITY);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) mx = fmaxf(mx, __uint_as_float(r[i]));
+                    for (int i = 0; i < 32; ++i)
+                        if (!(i <= lh && (!kWin || i >= ll))) r[half][i] = 0xFF800000u;      // -inf
                 }
             }
-            // the previous P V product must be done before P is overwritten or O is rescaled
-            if (j > 0 && !mbar_wait(bar_o_full, (j - 1) & 1, abort_flag, p.status)) { ok = false; break; }
+            float mx4[4] = {m_ref, m_ref, m_ref, m_ref};
+#pragma unroll
+            for (int i = 0; i < 64; i += 4)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) mx4[q] = fmaxf(mx4[q], __uint_as_float(r[i >> 5][(i & 31) + q]));
+            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
             const bool grow = (mx - m_ref) * c > 8.f;   // also true on the first tile (m_ref = -inf)
+            bool product_done = j == 0;
             if (__any_sync(0xffffffffu, grow)) {
                 // a row whose keys so far all lie left of its window has seen nothing yet (both maxima are -inf):
                 // it keeps its empty state instead of scaling by exp2(-inf + inf)
                 const float alpha = (kWin && mx == -INFINITY) ? 1.f : fast_exp2((m_ref - mx) * c);
                 if (j > 0) {
+                    // O is rescaled: the previous P V product must be done. Otherwise its completion is waited for below, behind
+                    // the exponentials (P goes over this tile's own scores, which that product does not read).
+                    if (!mbar_wait(bar_o_full, (j - 1) & 1, abort_flag, p.status)) { ok = false; break; }
+                    product_done = true;
                     tc_fence_after();
 #pragma unroll 1
                     for (int cc = 0; cc < 128; cc += 32) {
-                        uint32_t r[32];
-                        tmem_ld_32x32(tO + lane_base + cc, r);
+                        uint32_t o[32];
+                        tmem_ld_32x32(tO + lane_base + cc, o);
                         tmem_ld_wait();
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
-                        tmem_st_32x32(tO + lane_base + cc, r);
+                        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                        tmem_st_32x32(tO + lane_base + cc, o);
                     }
                     tmem_st_wait();
                 }
@@ -1777,39 +1819,36 @@ attn_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 m_ref = mx;
             }
             const float mc = m_ref * c;
-            float rs = 0.f;
-#pragma unroll 1
-            for (int half = 0; half < 2; ++half) {
-                uint32_t r[32];
-                tmem_ld_32x32(tSj + lane_base + half * 32, r);   // second read of the tile: cheaper than 64 live registers
-                tmem_ld_wait();
-                uint32_t pk[16];
-                // the row sum is taken from the fp32 probabilities (their bf16 roundings, which the P V product reads,
-                // differ from them by unbiased noise of relative size 2^-9 that averages out over a row)
-                if (need_mask) {
-                    const int lh = lim - half * 32, ll = lo - half * 32;
+            float rs4[4] = {0.f, 0.f, 0.f, 0.f};
+            // the row sum is taken from the fp32 probabilities (their bf16 roundings, which the P V product reads,
+            // differ from them by unbiased noise of relative size 2^-9 that averages out over a row)
+            auto probabilities = [&](auto masked) {
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    uint32_t pk[16];
 #pragma unroll
                     for (int i = 0; i < 32; i += 2) {
-                        const float e0 = fast_exp2(__uint_as_float(r[i]) * c - mc);
-                        const float e1 = fast_exp2(__uint_as_float(r[i + 1]) * c - mc);
-                        const float p0 = (i <= lh && (!kWin || i >= ll)) ? e0 : 0.f;
-                        const float p1 = (i + 1 <= lh && (!kWin || i + 1 >= ll)) ? e1 : 0.f;
+                        const float2 x = fma2(make_float2(__uint_as_float(r[half][i]), __uint_as_float(r[half][i + 1])), c, -mc);
+                        float p0 = fast_exp2(x.x), p1 = fast_exp2(x.y);
+                        if constexpr (decltype(masked)::value) {
+                            if (r[half][i] == 0xFF800000u) p0 = 0.f;
+                            if (r[half][i + 1] == 0xFF800000u) p1 = 0.f;
+                        }
                         pk[i >> 1] = pack_bf16(p0, p1);
-                        rs += p0 + p1;
+                        rs4[i & 2] += p0;
+                        rs4[(i & 2) + 1] += p1;
                     }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 32; i += 2) {
-                        const float p0 = fast_exp2(__uint_as_float(r[i]) * c - mc);
-                        const float p1 = fast_exp2(__uint_as_float(r[i + 1]) * c - mc);
-                        pk[i >> 1] = pack_bf16(p0, p1);
-                        rs += p0 + p1;
-                    }
+                    tmem_st_32x16(tSj + lane_base + half * 16, pk);      // P over the first 32 columns of this score buffer
                 }
-                tmem_st_32x16(tSj + lane_base + half * 16, pk);      // P over the first 32 columns of this score buffer
-            }
+            };
+            if (need_mask) probabilities(std::true_type{});
+            else probabilities(std::false_type{});
+            const float rs = (rs4[0] + rs4[1]) + (rs4[2] + rs4[3]);
             tmem_st_wait();
             l += rs;
+            // every phase of the barrier is waited for in turn, and before this tile's product can complete the next one: a
+            // parity would not tell two phases apart
+            if (!product_done && !mbar_wait(bar_o_full, (j - 1) & 1, abort_flag, p.status)) { ok = false; break; }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_p_ready);
@@ -1900,12 +1939,12 @@ static int launch_fwd3_sinks(const CUtensorMap& tq, const CUtensorMap& tk, const
                              int n_tiles, cudaStream_t stream) {
     static bool cfg = false;
     if (!cfg) {
-        if (set_smem((const void*)attn_fwd3_kernel<false, kWin>, kFwd2Smem)) return -10;
+        if (set_smem((const void*)attn_fwd3_kernel<false, kWin>, kFwd3Smem)) return -10;
         cudaFuncSetAttribute((const void*)attn_fwd3_kernel<false, kWin>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              cudaSharedmemCarveoutMaxShared);
         cfg = true;
     }
-    attn_fwd3_kernel<false, kWin><<<dim3(p.Hq, n_tiles), kFwdThreads, kFwd2Smem, stream>>>(tq, tk, tv, p, g_no_cp_args);
+    attn_fwd3_kernel<false, kWin><<<dim3(p.Hq, n_tiles), kFwdThreads, kFwd3Smem, stream>>>(tq, tk, tv, p, g_no_cp_args);
     return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
@@ -1967,13 +2006,13 @@ int halo_attn_fwd3(const void* q, const void* k, const void* v, void* o, float* 
     if (make_tmap_bf16(&tv, v, T, (long long)Hkv * kHd, ldv, 64)) return -4;
     static bool cfg = false;
     if (!cfg) {
-        if (set_smem((const void*)attn_fwd3_kernel<false>, kFwd2Smem)) return -10;
+        if (set_smem((const void*)attn_fwd3_kernel<false>, kFwd3Smem)) return -10;
         cudaFuncSetAttribute((const void*)attn_fwd3_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              cudaSharedmemCarveoutMaxShared);
         cfg = true;
     }
     AttnParams p{reinterpret_cast<const FwdWork*>(work), o, lse, ldo, T, Hq, Hkv, scale, status};
-    attn_fwd3_kernel<false><<<dim3(Hq, n_tiles), kFwdThreads, kFwd2Smem, (cudaStream_t)stream>>>(tq, tk, tv, p, g_no_cp_args);
+    attn_fwd3_kernel<false><<<dim3(Hq, n_tiles), kFwdThreads, kFwd3Smem, (cudaStream_t)stream>>>(tq, tk, tv, p, g_no_cp_args);
     return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
@@ -1990,13 +2029,13 @@ int halo_attn_fwd3_window(const void* q, const void* k, const void* v, void* o, 
     if (make_tmap_bf16(&tv, v, T, (long long)Hkv * kHd, ldv, 64)) return -4;
     static bool cfg = false;
     if (!cfg) {
-        if (set_smem((const void*)attn_fwd3_kernel<false, true>, kFwd2Smem)) return -10;
+        if (set_smem((const void*)attn_fwd3_kernel<false, true>, kFwd3Smem)) return -10;
         cudaFuncSetAttribute((const void*)attn_fwd3_kernel<false, true>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              cudaSharedmemCarveoutMaxShared);
         cfg = true;
     }
     AttnParams p{reinterpret_cast<const FwdWork*>(work), o, lse, ldo, T, Hq, Hkv, scale, status, window};
-    attn_fwd3_kernel<false, true><<<dim3(Hq, n_tiles), kFwdThreads, kFwd2Smem, (cudaStream_t)stream>>>(tq, tk, tv, p, g_no_cp_args);
+    attn_fwd3_kernel<false, true><<<dim3(Hq, n_tiles), kFwdThreads, kFwd3Smem, (cudaStream_t)stream>>>(tq, tk, tv, p, g_no_cp_args);
     return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
@@ -2073,13 +2112,13 @@ int halo_attn_cp_fwd(const void* q, void* const* kv_ptrs, int n_ranks, long long
     if (fill_cp_map(&ca.cp, cp_map, 8) || fill_cp_map(&ca.cpk, kv_map, n_ranks)) return -4;
     static bool cfg = false;
     if (!cfg) {
-        if (set_smem((const void*)attn_fwd3_kernel<true>, kFwd2Smem)) return -10;
+        if (set_smem((const void*)attn_fwd3_kernel<true>, kFwd3Smem)) return -10;
         cudaFuncSetAttribute((const void*)attn_fwd3_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              cudaSharedmemCarveoutMaxShared);
         cfg = true;
     }
     AttnParams p{reinterpret_cast<const FwdWork*>(work), o, lse, ldo, T_local, Hq, Hkv, scale, status};
-    attn_fwd3_kernel<true><<<dim3(Hq, n_tiles), kFwdThreads, kFwd2Smem, (cudaStream_t)stream>>>(tq, ca.peers.k[0], ca.peers.v[0], p, ca);
+    attn_fwd3_kernel<true><<<dim3(Hq, n_tiles), kFwdThreads, kFwd3Smem, (cudaStream_t)stream>>>(tq, ca.peers.k[0], ca.peers.v[0], p, ca);
     return cudaGetLastError() == cudaSuccess ? 0 : -11;
 }
 
