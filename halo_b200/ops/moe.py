@@ -122,6 +122,7 @@ class LocalTransport:
 
     n_ranks = 1
     rank = 0
+    plan_locally = True      # one planning launch instead of the handshake and the plans of the general path
 
     def __init__(self, capacity_factor: float = 1.0):
         from halo_b200 import env
@@ -405,14 +406,86 @@ def _fused(transport) -> bool:
     return bool(getattr(transport, "fused", False)) and hasattr(transport, "ctrl_table")
 
 
+def _list_spec(gated: int, n_cols: int, k_dim: int, b_mn_stride: int, b_k_stride: int, swiglu_f: int = 0):
+    """Key of a tile list in a routing state, and the column tiles of the product."""
+    tile_n, width = (128, swiglu_f) if swiglu_f else (256, n_cols)
+    return ("ep", gated, n_cols, k_dim, b_mn_stride, b_k_stride, swiglu_f), (width + tile_n - 1) // tile_n
+
+
+def _plan_local(counts, capacity: int, specs, H: int, arrive, buf, meta, row_w, layout=None, units=None):
+    """One launch on one rank: the tile lists of two products (their specs as in :func:`_list_spec`), zeroed arrival
+    counters, pad rows, and - with ``layout`` / ``units`` - the receive layout and push units. Returns the lists by key."""
+    dev = counts.device
+    L = _lib.lib()
+    out, args, ptrs = {}, [], []
+    sizes = [max(capacity // 128, 1) * tiles_n for _, tiles_n in specs]
+    wb = _work_bytes()
+    lists = torch.empty(sum(sizes) * wb, dtype=torch.uint8, device=dev)
+    marks = torch.empty(2, dtype=torch.int32, device=dev)
+    at = 0
+    for i, ((key, tiles_n), n) in enumerate(zip(specs, sizes)):
+        lst, count = lists[at * wb:(at + n) * wb], marks[i:i + 1]
+        at += n
+        out[key] = (lst, count, tiles_n)
+        args += [key[2], key[3], key[4], key[5], key[6], key[1], n]
+        ptrs += [_lib.ptr(lst), _lib.ptr(count)]
+    layout = [_lib.ptr(t) for t in layout] if layout is not None else [_lib.c_void_p(0)] * 5
+    units = ([_lib.ptr(units[0]), _lib.ptr(units[1]), _lib.c_int(units[2])] if units is not None
+             else [_lib.c_void_p(0), _lib.c_void_p(0), _lib.c_int(0)])
+    rc = L.halo_moe_plan_local(_lib.ptr(counts), _lib.c_int(counts.numel()), _lib.c_int(H), *layout, *units, _lib.c_void_p(arrive[0]),
+                               _lib.ptr(buf), _lib.ptr(meta), _lib.ptr(row_w), *ptrs, (_lib.c_int * 14)(*args),
+                               _lib.stream_ptr(dev))
+    _lib.check(rc, "halo_moe_plan_local")
+    return out
+
+
+def _local_plan_ok(transport, n_slots: int, n_experts: int, capacity: int) -> bool:
+    """One rank whose buffer no routing can overflow."""
+    return getattr(transport, "plan_locally", False) and transport.n_ranks == 1 and capacity >= n_slots + 127 * n_experts
+
+
+def _plan_routing_local(topk_idx, n_experts: int, transport, specs, H: int, buf, meta) -> RoutingState:
+    """What :func:`plan_routing_fused` and the first pad zeroing give on one rank, from one planning launch. ``buf``: the
+    receive buffer whose pad rows are to be zero (None: nobody will read them)."""
+    T, k = topk_idx.shape
+    n_slots = T * k
+    dev = topk_idx.device
+    L = _lib.lib()
+    capacity = transport.capacity(n_slots, n_experts)
+    transport.prepare_ctrl(n_experts, capacity, dev)
+    idx = topk_idx.contiguous()
+    n_blocks = L.halo_route_blocks(_lib.c_ll(n_slots))
+    ints = torch.empty(max(n_blocks, 1) * n_experts + 5 * n_experts + 2 + 2 * n_slots, dtype=torch.int32, device=dev)
+    block_hist, counts, seg_start, seg_rows, dst_base, my_prefix, total_rows, n_units, slot_row, send_slot = ints.split(
+        [max(n_blocks, 1) * n_experts, n_experts, n_experts, n_experts, n_experts, n_experts, 1, 1, n_slots, n_slots])
+    s = _lib.stream_ptr(dev)
+    _lib.check(L.halo_route_count(_lib.ptr(idx), _lib.c_ll(n_slots), _lib.c_int(n_experts), _lib.ptr(block_hist),
+                                  _lib.ptr(counts), s), "halo_route_count")
+    seq = transport.next_seq()
+    max_units = n_slots // 128 + 2 * n_experts + 2
+    units = torch.empty(max_units * int(L.halo_moe_push_unit_bytes()), dtype=torch.uint8, device=dev)
+    lists = _plan_local(counts, capacity, specs, H, transport.arrive_table(seq), buf, meta, None,
+                        (seg_start, seg_rows, dst_base, my_prefix, total_rows), (units, n_units, max_units))
+    _lib.check(L.halo_route_place_send(_lib.ptr(idx), _lib.c_ll(n_slots), _lib.c_int(n_experts), _lib.ptr(block_hist),
+                                       _lib.ptr(dst_base), _lib.ptr(slot_row), _lib.ptr(my_prefix), _lib.ptr(send_slot), s),
+               "halo_route_place_send")
+    return RoutingState(n_tokens=T, top_k=k, n_experts=n_experts, n_local=n_experts, capacity=capacity, topk_idx=idx,
+                        slot_row=slot_row, seg_start=seg_start, seg_rows=seg_rows, total_rows=total_rows, counts=counts,
+                        lists=lists, send_slot=send_slot, units=units, n_units=n_units, seq=seq)
+
+
+def _check_fused_size(n_slots: int, n_experts: int) -> None:
+    if n_slots >= 1 << 24 or n_experts > 256:
+        raise ValueError(f"the fused expert path tags rows with 24-bit slot numbers and plans up to 256 experts "
+                         f"(got {n_slots} slots, {n_experts} experts); set HALO_MOE_FUSED=0 for larger calls")
+
+
 def plan_routing_fused(topk_idx: torch.Tensor, n_experts: int, transport) -> RoutingState:
     """Routing state of one call on the fused path: this rank's histogram, the handshake that hands it to every peer
     and derives every receive layout, slot placement with the destination-ordered send list, the push units and the
     receive-buffer tiles in arrival order. All on the device; nothing is read back."""
     T, k = topk_idx.shape
-    if T * k >= 1 << 24 or n_experts > 256:
-        raise ValueError(f"the fused expert path tags rows with 24-bit slot numbers and plans up to 256 experts "
-                         f"(got {T * k} slots, {n_experts} experts); set HALO_MOE_FUSED=0 for larger calls")
+    _check_fused_size(T * k, n_experts)
     n_ranks, me = transport.n_ranks, transport.rank
     n_local = n_experts // n_ranks
     capacity = transport.capacity(T * k, n_local)
@@ -462,22 +535,20 @@ def plan_routing_fused(topk_idx: torch.Tensor, n_experts: int, transport) -> Rou
 
 def _ep_list(state: RoutingState, gated: int, n_cols: int, k_dim: int, b_mn_stride: int, b_k_stride: int, swiglu_f: int = 0):
     """Tile list of one grouped product over the receive-buffer tiles in arrival order (cached per routing state)."""
-    key = ("ep", gated, n_cols, k_dim, b_mn_stride, b_k_stride, swiglu_f)
+    key, tiles_n = _list_spec(gated, n_cols, k_dim, b_mn_stride, b_k_stride, swiglu_f)
     hit = state.lists.get(key)
     if hit is not None:
         return hit
     L = _lib.lib()
     dev = state.slot_row.device
-    tile_n = 128 if swiglu_f else 256
-    width = swiglu_f if swiglu_f else n_cols
-    max_items = max(state.capacity // 128, 1) * ((width + tile_n - 1) // tile_n)
+    max_items = max(state.capacity // 128, 1) * tiles_n
     lst = torch.empty(max_items * _work_bytes(), dtype=torch.uint8, device=dev)
     count = torch.empty(1, dtype=torch.int32, device=dev)
     _lib.check(L.halo_moe_plan_items(_lib.ptr(state.tiles), _lib.ptr(state.n_tiles), _lib.c_int(n_cols), _lib.c_int(k_dim),
                                      _lib.c_int(b_mn_stride), _lib.c_int(b_k_stride), _lib.c_int(swiglu_f), _lib.c_int(gated),
                                      _lib.ptr(lst), _lib.ptr(count), _lib.c_int(max_items), _lib.stream_ptr(dev)),
                "halo_moe_plan_items")
-    state.lists[key] = (lst, count, (width + tile_n - 1) // tile_n)
+    state.lists[key] = (lst, count, tiles_n)
     return state.lists[key]
 
 
@@ -534,12 +605,21 @@ def _fused_forward(ctx, x, topk_idx, topk_w, w_gate_up, w_down, transport, state
     k = topk_idx.shape[1]
     dev = x.device
     _mark("start", dev)
-    state = plan_routing_fused(topk_idx, n_experts, transport)
-    cap = state.capacity
-    recv_x = transport.buffer("recv_x", cap, H, torch.bfloat16, dev)
-    meta = transport.buffer("row_meta", cap, 1, torch.int32, dev)
-    _zero_pads(state, recv_x, meta, None)
+    _check_fused_size(T * k, n_experts)
     need_grad = grad_mode and any(ctx.needs_input_grad)
+    cap = transport.capacity(T * k, E_local)
+    if _local_plan_ok(transport, T * k, n_experts, cap):
+        recv_x = transport.buffer("recv_x", cap, H, torch.bfloat16, dev)
+        meta = transport.buffer("row_meta", cap, 1, torch.int32, dev)
+        # pad rows are read by nobody but the weight gradients: their products' rows go nowhere
+        state = _plan_routing_local(topk_idx, n_experts, transport, (_list_spec(1, F2, H, F2, 0, F), _list_spec(0, H, F, H, 0)), H,
+                                    recv_x if need_grad else None, meta)
+    else:
+        state = plan_routing_fused(topk_idx, n_experts, transport)
+        cap = state.capacity
+        recv_x = transport.buffer("recv_x", cap, H, torch.bfloat16, dev)
+        meta = transport.buffer("row_meta", cap, 1, torch.int32, dev)
+        _zero_pads(state, recv_x, meta, None)
     act = _alloc(transport, (cap, F), torch.bfloat16, dev)
     pre = _alloc(transport, (cap, F2), torch.bfloat16, dev) if need_grad else None
     lst1 = _ep_list(state, 1, F2, H, F2, 0, F)
@@ -583,15 +663,23 @@ def _fused_backward(ctx, dout):
     n_ranks, me = transport.n_ranks, transport.rank
     _mark("start", dev)
     # 1. a handshake of its own: every rank is done with the buffers of its previous call, the arrival counters restart
+    local = state.tiles is None        # planned in one launch on one rank
+    if local:
+        transport.prepare_ctrl(state.n_experts, cap, dev)
     seq = transport.next_seq()
-    _lib.check(L.halo_moe_handshake(transport.ctrl_table(), _lib.c_int(me), _lib.c_int(n_ranks), _lib.c_int(state.n_experts),
-                                    _lib.c_int(seq), _lib.c_int(transport.max_tiles), _lib.c_void_p(0), _lib.c_int(cap),
-                                    _lib.c_void_p(0), _lib.c_void_p(0), _lib.c_void_p(0), _lib.c_void_p(0), _lib.c_void_p(0),
-                                    _lib.ptr(_lib.status_word(dev)), s), "halo_moe_handshake")
+    if not local:
+        _lib.check(L.halo_moe_handshake(transport.ctrl_table(), _lib.c_int(me), _lib.c_int(n_ranks), _lib.c_int(state.n_experts),
+                                        _lib.c_int(seq), _lib.c_int(transport.max_tiles), _lib.c_void_p(0), _lib.c_int(cap),
+                                        _lib.c_void_p(0), _lib.c_void_p(0), _lib.c_void_p(0), _lib.c_void_p(0), _lib.c_void_p(0),
+                                        _lib.ptr(_lib.status_word(dev)), s), "halo_moe_handshake")
     dy = transport.buffer("recv_dy", cap, H, torch.bfloat16, dev)
     row_w = transport.buffer("row_w", cap, 1, torch.float32, dev)
     meta = transport.buffer("row_meta", cap, 1, torch.int32, dev)
-    _zero_pads(state, dy, meta, row_w)
+    if local:
+        state.lists.update(_plan_local(state.counts, cap, (_list_spec(1, F, H, 0, H), _list_spec(0, H, F2, 0, F2)), H,
+                                       transport.arrive_table(seq), dy, meta, row_w))
+    else:
+        _zero_pads(state, dy, meta, row_w)
     # 2. dout rows (with their routing weights) travel to the experts inside the first product:
     #    dact_u = dout_rows W_down (unscaled activation gradient)
     dact = _alloc(transport, (cap, F), torch.bfloat16, dev)

@@ -232,3 +232,36 @@ def test_grouped_products_over_uneven_experts(pair, E, T, H, F):
         assert ((z[s:s + n] - want).abs() <= 2.0 ** -8 * want.abs() + 1e-3).all(), e
         assert (z[s + n:s + (n + 127) // 128 * 128] == 0).all()
     assert _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("T,H,F,E,k", [(1, 256, 128, 8, 1), (32, 512, 256, 128, 8), (129, 256, 136, 5, 3), (2050, 512, 256, 256, 4)])
+def test_one_launch_plan_equals_the_general_path(T, H, F, E, k):
+    """The plan of a single-rank call against handshake, push, tile, item and pad kernels: outputs, gradients and the layout
+    bit for bit, with empty experts, one expert that takes a slot of every token, and calls with and without gradients."""
+    from halo_b200.ops import _lib
+    from halo_b200.ops.moe import LocalTransport, moe_experts
+
+    torch.manual_seed(T)
+    x = torch.randn(T, H, device="cuda").bfloat16()
+    scores = torch.rand(T, E, device="cuda")
+    scores[:, 1] = 0.0
+    scores[:, 0] = 2.0
+    w, idx = torch.topk(scores, k, dim=-1)
+    idx = idx.to(torch.int32)
+    wgu, wd = (torch.randn(E, 2 * F, H, device="cuda") * 0.05).bfloat16(), (torch.randn(E, H, F, device="cuda") * 0.05).bfloat16()
+    g = torch.randn(T, H, device="cuda").bfloat16()
+    results = []
+    for locally in (True, False):
+        transport = LocalTransport()
+        transport.fused, transport.plan_locally = True, locally
+        states = []
+        with torch.no_grad():
+            plain = moe_experts(x, idx, w, wgu, wd, transport, state_out=states)
+        leaves = [t.clone().requires_grad_() for t in (x, w, wgu, wd)]
+        out = moe_experts(leaves[0], idx, leaves[1], leaves[2], leaves[3], transport, state_out=states)
+        grads = torch.autograd.grad(out, leaves, g)
+        layout = [getattr(s, n) for s in states for n in ("seg_start", "seg_rows", "total_rows", "counts", "slot_row", "send_slot", "n_units")]
+        results.append([plain, out.detach(), *grads, *layout])
+        assert (states[0].tiles is None) == locally and _lib.read_status() == 0
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
