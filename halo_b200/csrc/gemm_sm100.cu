@@ -357,6 +357,21 @@ int make_tmap_bf16(CUtensorMap* m, const void* base, long long rows, long long c
     return 0;
 }
 
+// Output map of the wide kernel: 32 rows x 128 bytes, rows `ld` elements apart, as many as a launch can name.
+static int make_tmap_out(CUtensorMap* m, void* base, long long ld, bool f32) {
+    EncodeTiledFn fn = get_encode_fn();
+    const int bytes = f32 ? 4 : 2;
+    if (!fn || (reinterpret_cast<uintptr_t>(base) & 15u) || (ld * bytes) % 16 || ld <= 0) return -2;
+    cuuint64_t dims[2] = {(cuuint64_t)ld, (cuuint64_t)1 << 30};
+    cuuint64_t strides[1] = {(cuuint64_t)ld * bytes};
+    cuuint32_t box[2] = {128u / bytes, 32u};
+    cuuint32_t estr[2] = {1u, 1u};
+    const CUresult r = fn(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? 0 : -3;
+}
+
 static int g_num_sms = 0;
 static int num_sms() {
     if (!g_num_sms) {
@@ -441,7 +456,8 @@ static int launch_few_rows(const void* X, const void* W, long long ldx, long lon
 }
 
 template <bool A_MN, bool B_MN>
-static int launch_wide_t(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int n_pairs, cudaStream_t stream) {
+static int launch_wide_t(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const CUtensorMap& tx,
+                         const GemmParams& p, int n_pairs, cudaStream_t stream) {
     static bool configured = false;
     if (!configured) {
         if (cudaFuncSetAttribute(gemm_wide_kernel<A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideSmemBytes) != cudaSuccess)
@@ -460,14 +476,20 @@ static int launch_wide_t(const CUtensorMap& ta, const CUtensorMap& tb, const Gem
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, gemm_wide_kernel<A_MN, B_MN>, ta, tb, p) == cudaSuccess ? 0 : -11;
+    return cudaLaunchKernelEx(&cfg, gemm_wide_kernel<A_MN, B_MN>, ta, tb, tc, tx, p) == cudaSuccess ? 0 : -11;
 }
 
-static int launch_wide(int a_mn, int b_mn, const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int n_pairs, cudaStream_t s) {
-    if (!a_mn && !b_mn) return launch_wide_t<false, false>(ta, tb, p, n_pairs, s);
-    if (!a_mn && b_mn) return launch_wide_t<false, true>(ta, tb, p, n_pairs, s);
-    if (a_mn && b_mn) return launch_wide_t<true, true>(ta, tb, p, n_pairs, s);
-    return launch_wide_t<true, false>(ta, tb, p, n_pairs, s);
+static int launch_wide(int a_mn, int b_mn, const CUtensorMap& ta, const CUtensorMap& tb, GemmParams p, int n_pairs, cudaStream_t s) {
+    // Only whole 32-row blocks of 128 bytes go through these maps, so their extents need not be the tensors' (a list names rows
+    // of a bank whose height is not passed); a base or stride that cannot be encoded leaves the stores to the lanes.
+    CUtensorMap tc{}, tx{};
+    const bool f32 = p.epi == kEpiStoreF32 || p.epi == kEpiAccumF32;
+    if (p.epi != kEpiAccumBf16) p.tma_c = make_tmap_out(&tc, p.C, p.ldc, f32) == 0;
+    if (p.epi == kEpiSwiglu && p.aux) p.tma_aux = make_tmap_out(&tx, p.aux, p.ld_aux, false) == 0;
+    if (!a_mn && !b_mn) return launch_wide_t<false, false>(ta, tb, tc, tx, p, n_pairs, s);
+    if (!a_mn && b_mn) return launch_wide_t<false, true>(ta, tb, tc, tx, p, n_pairs, s);
+    if (a_mn && b_mn) return launch_wide_t<true, true>(ta, tb, tc, tx, p, n_pairs, s);
+    return launch_wide_t<true, false>(ta, tb, tc, tx, p, n_pairs, s);
 }
 
 // Work items of a dense product: whole 256 x 512 tiles for the full waves of pairs; a last wave that would leave more than

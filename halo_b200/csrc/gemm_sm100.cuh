@@ -66,6 +66,7 @@ struct GemmParams {
     void* c_peers[8];
     int rs_ranks, rs_rank, rs_rows;
     int wide_full, wide_items;   // gemm_wide_kernel, dense: whole tiles, and work items with the column halves that follow them
+    int tma_c, tma_aux;          // gemm_wide_kernel: whole blocks of C / of the pre-activations are stored by TMA
     // kEpiClampedGlu: bias bank as one bf16 vector indexed like the rows of B, the clamp and the gate's slope
     const void* glu_bias;
     float glu_limit, glu_alpha;

@@ -9,11 +9,11 @@
 // (ncu, 8192 x 8192 x 4096). Sharing A between two column blocks brings that to 48 + 64 KB per 1,024 cycles and takes a
 // quarter of the L2 traffic away. Measured under the power cap (0.5 s loops, bf16, TFLOP/s; before = the better of 128 x 256
 // single-CTA and 256 x 256 pair tiles / now):
-//   8192 x 24576 x 4096 (y = x W^T)      1142 / 1298     24576 x 4096 x 8192 (dy^T x)    1176 / 1357
-//   8192 x 4096 x 12288 (y = x W^T)      1177 / 1346     4096 x 12288 x 8192 (dy^T x)    1134 / 1313
-//   8192 x 4096 x 24576 (dy W)           1200 / 1369     4096 x 151936 x 2048 (logits)   1079 / 1265
-//   8192 x 12288 x 4096 (dy W)           1163 / 1309     4096 x 2048 x 151936 (dlogits W) 1153 / 1367
-//   151936 x 2048 x 4096, fp32 +=        1005 / 1227     SwiGLU 8192 x 24576 x 4096      1096 / 1255
+//   8192 x 24576 x 4096 (y = x W^T)      1142 / 1302     24576 x 4096 x 8192 (dy^T x)    1176 / 1380
+//   8192 x 4096 x 12288 (y = x W^T)      1177 / 1378     4096 x 12288 x 8192 (dy^T x)    1134 / 1332
+//   8192 x 4096 x 24576 (dy W)           1200 / 1400     4096 x 151936 x 2048 (logits)   1079 / 1277
+//   8192 x 12288 x 4096 (dy W)           1163 / 1337     4096 x 2048 x 151936 (dlogits W) 1153 / 1384
+//   151936 x 2048 x 4096, fp32 +=        1005 / 1268     SwiGLU 8192 x 24576 x 4096      1096 / 1287
 //
 // Tensor memory holds no second tile, so the epilogue is kept off the critical path differently. The two column blocks are
 // two accumulators with barriers of their own: all eight epilogue warps take block 0 into registers first, and the next
@@ -140,20 +140,68 @@ __device__ __forceinline__ void wide_take_bf16(uint32_t t_addr, float alpha, boo
             pk[16 * c + j] = zero ? 0u : pack_bf16(__uint_as_float(r[2 * j]) * alpha, __uint_as_float(r[2 * j + 1]) * alpha);
     }
 }
-// ... and goes to columns col0 .. of the tile, 64 at a time, `dst` being the tile's column 0 of this warp's first row
+// Where a warp's rows go: by TMA (`map`, with the warp's first row and the tile's column 0 in C) where a whole 32-row block of
+// 128 bytes exists, else by the lanes. Ordinary stores from the transposition buffer - four 128-byte pieces an instruction -
+// take longer than the products they follow once the reduction is short: weight gradients of experts with 190 rows, 805 MB of
+// them, took 332 us that way, 198 us without the stores and 305 us by TMA.
+struct WideOut {
+    const CUtensorMap* map;     // null: the lanes store
+    void* base;                 // the warp's first row, column 0 of the tile
+    long long ld;
+    int row, col;               // coordinates of `base` in the map
+    int rows, n_valid;          // rows of this warp that exist, columns of the tile
+    uint32_t stage;
+    int lane;
+};
+
+// 128 bytes of the warp's 32 rows to columns col .. of the tile (`col` counted in elements of BYTES bytes)
+template <int BYTES, bool ADD>
+__device__ __forceinline__ void wide_put_row_block(const WideOut& o, const uint32_t (&v)[32], int col) {
+    constexpr int kUnit = 16 / BYTES, kCols = 128 / BYTES;
+    if (o.map && o.rows == 32 && col + kCols <= o.n_valid) {        // uniform over the warp
+        if (o.lane == 0) tma_store_wait_read<0>();                  // the buffer's previous block has been read
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(o.stage + o.lane * 128 + ((u ^ (o.lane & 7)) << 4)),
+                         "r"(v[4 * u]), "r"(v[4 * u + 1]), "r"(v[4 * u + 2]), "r"(v[4 * u + 3])
+                         : "memory");
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (o.lane == 0) {
+            if (ADD) tma_reduce_add_2d(o.map, o.stage, o.col + col, o.row);
+            else tma_store_2d(o.map, o.stage, o.col + col, o.row);
+            tma_store_commit();
+        }
+        return;
+    }
+    if (o.map) {                                                    // the lanes take over a buffer that TMA may still read
+        if (o.lane == 0) tma_store_wait_read<0>();
+        __syncwarp();
+    }
+    through_smem(o.stage, o.lane, v, [&](int rr, int u, uint4 x) {
+        const int c = col + u * kUnit;
+        if (rr >= o.rows || c + kUnit > o.n_valid) return;
+        uint8_t* d = reinterpret_cast<uint8_t*>(o.base) + ((long long)rr * o.ld + c) * BYTES;
+        if (ADD) {
+            const float4 c0 = *reinterpret_cast<const float4*>(d);
+            *reinterpret_cast<float4*>(d) = make_float4(c0.x + __uint_as_float(x.x), c0.y + __uint_as_float(x.y),
+                                                        c0.z + __uint_as_float(x.z), c0.w + __uint_as_float(x.w));
+        } else {
+            *reinterpret_cast<uint4*>(d) = x;
+        }
+    });
+}
+
 template <int N64>
-__device__ __forceinline__ void wide_put_bf16(__nv_bfloat16* dst, long long ld, const uint32_t (&pk)[32 * N64], int col0, int n_valid, int rows,
-                                              uint32_t stage, int lane) {
+__device__ __forceinline__ void wide_put_bf16(const WideOut& o, const uint32_t (&pk)[32 * N64], int col0) {
 #pragma unroll
     for (int h = 0; h < N64; ++h) {
-        if (col0 + 64 * h >= n_valid) break;                       // uniform over the warp
+        if (col0 + 64 * h >= o.n_valid) break;                     // uniform over the warp
         uint32_t v[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = pk[32 * h + j];
-        through_smem(stage, lane, v, [&](int rr, int u, uint4 x) {
-            const int col = col0 + 64 * h + u * 8;
-            if (rr < rows && col + 8 <= n_valid) *reinterpret_cast<uint4*>(dst + (long long)rr * ld + col) = x;
-        });
+        wide_put_row_block<2, false>(o, v, col0 + 64 * h);
     }
 }
 __device__ __forceinline__ void wide_take_f32(uint32_t t_addr, float alpha, bool zero, uint32_t (&v)[2][32]) {
@@ -165,24 +213,15 @@ __device__ __forceinline__ void wide_take_f32(uint32_t t_addr, float alpha, bool
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[c][j] = zero ? 0u : __float_as_uint(__uint_as_float(v[c][j]) * alpha);
 }
-// fp32 output; accumulation is a vector reduction in L2: every element receives exactly one addition per launch, so the
-// result is that of a load, an addition and a store, without the wait for the load
-__device__ __forceinline__ void wide_put_f32(float* dst, long long ld, const uint32_t (&v)[2][32], bool accumulate, int col0, int n_valid,
-                                             int rows, uint32_t stage, int lane) {
+// fp32 output; accumulation of whole blocks is a TMA reduction in L2: every element receives exactly one addition per launch,
+// so the result is that of a load, an addition and a store, without the wait for the load. Subnormal sums survive it, which
+// they do not in `red.global.add.f32`.
+template <bool ADD>
+__device__ __forceinline__ void wide_put_f32(const WideOut& o, const uint32_t (&v)[2][32], int col0) {
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
-        if (col0 + 32 * c >= n_valid) break;
-        through_smem(stage, lane, v[c], [&](int rr, int u, uint4 x) {
-            const int col = col0 + 32 * c + u * 4;
-            if (rr >= rows || col + 4 > n_valid) return;
-            float* d = dst + (long long)rr * ld + col;
-            if (accumulate)
-                asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(d), "f"(__uint_as_float(x.x)),
-                             "f"(__uint_as_float(x.y)), "f"(__uint_as_float(x.z)), "f"(__uint_as_float(x.w))
-                             : "memory");
-            else
-                *reinterpret_cast<uint4*>(d) = x;
-        });
+        if (col0 + 32 * c >= o.n_valid) break;
+        wide_put_row_block<4, ADD>(o, v[c], col0 + 32 * c);
     }
 }
 // bf16 output += tile: the sum is formed in fp32 and rounded once
@@ -211,6 +250,7 @@ __device__ __forceinline__ void wide_add_bf16(__nv_bfloat16* dst, long long ld, 
 template <bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(kWideThreads, 1)
 gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                 const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmAux,
                  const __grid_constant__ GemmParams p) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t bar_full[kWideStages], bar_empty[kWideStages], bar_tfull[2], bar_tempty[2];
@@ -338,6 +378,8 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                     issue(s0, 0, kb != 0);
                     if (++s0 == kWideStages) { s0 = 0; ph0 ^= 1u; }
                 }
+                // a short reduction: block 0 is complete, and its epilogue need not wait for the other block's turn
+                if (ok && w.k_iters <= ahead) wide_commit(smem_u32(&bar_tfull[0]));
                 if (!ok || !mbar_wait(smem_u32(&bar_tempty[1]), (used[1] & 1u) ^ 1u, &abort_flag, p.status)) break;
                 tc_fence_after();
                 ++used[1];
@@ -356,7 +398,6 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                     if (++stage == kWideStages) { stage = 0; phase ^= 1u; }
                 }
                 if (!ok) break;
-                if (w.k_iters <= ahead) wide_commit(smem_u32(&bar_tfull[0]));
                 wide_commit(smem_u32(&bar_tfull[1]));
             }
         }
@@ -388,6 +429,8 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             const int rows = max(0, min(32, w.m_valid - int(rank) * 128 - row0));       // rows of this warp that exist
             const long long c_row = (long long)w.c_row + int(rank) * 128 + row0;
             const bool zero = w.k_iters == 0;
+            WideOut out{p.tma_c ? &tmC : nullptr, nullptr, p.ldc, (int)c_row, w.c_col, rows, w.n_valid, stage, lane};
+            out.base = reinterpret_cast<uint8_t*>(p.C) + (c_row * p.ldc + w.c_col) * (f32 ? 4 : 2);
             if (wide_values) {
                 bool ok = true;
                 for (int block = 0; block < w.pad0; ++block) {
@@ -398,23 +441,24 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                         wide_take_f32(t_row + block * kBlockN + 64 * h, p.alpha, zero, v);
                         if (h == 1) release(block);
                         const int col0 = block * 256 + half * 128 + 64 * h;
-                        if (f32)
-                            wide_put_f32(reinterpret_cast<float*>(p.C) + c_row * p.ldc + w.c_col, p.ldc, v, p.epi == kEpiAccumF32, col0,
-                                         w.n_valid, rows, stage, lane);
-                        else
-                            wide_add_bf16(reinterpret_cast<__nv_bfloat16*>(p.C) + c_row * p.ldc + w.c_col, p.ldc, v, col0, w.n_valid, rows,
-                                          lane);
+                        if (p.epi == kEpiAccumF32) wide_put_f32<true>(out, v, col0);
+                        else if (f32) wide_put_f32<false>(out, v, col0);
+                        else wide_add_bf16(reinterpret_cast<__nv_bfloat16*>(out.base), p.ldc, v, col0, w.n_valid, rows, lane);
                     }
                 }
                 if (!ok) break;
                 continue;
             }
-            __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.C) + c_row * p.ldc + w.c_col;
             if (p.epi == kEpiSwiglu) {
                 // block 0 is the gate, block 1 the up half; both rounded to bf16 first, so that a recomputation from the saved
                 // pre-activations sees the same values
                 if (!ready(0) || !ready(1)) break;
-                __nv_bfloat16* pre = p.aux ? reinterpret_cast<__nv_bfloat16*>(p.aux) + c_row * p.ld_aux + w.c_col : nullptr;
+                WideOut gate = out, up = out;
+                gate.map = up.map = p.tma_aux ? &tmAux : nullptr;
+                gate.ld = up.ld = p.ld_aux;
+                gate.base = reinterpret_cast<__nv_bfloat16*>(p.aux) + c_row * p.ld_aux + w.c_col;
+                up.base = reinterpret_cast<__nv_bfloat16*>(gate.base) + p.swiglu_f;
+                up.col = w.c_col + p.swiglu_f;
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     uint32_t g[32], u[32];
@@ -425,9 +469,9 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                         release(1);
                     }
                     const int col0 = half * 128 + 64 * h;
-                    if (pre) {
-                        wide_put_bf16<1>(pre, p.ld_aux, g, col0, w.n_valid, rows, stage, lane);
-                        wide_put_bf16<1>(pre + p.swiglu_f, p.ld_aux, u, col0, w.n_valid, rows, stage, lane);
+                    if (p.aux) {
+                        wide_put_bf16<1>(gate, g, col0);
+                        wide_put_bf16<1>(up, u, col0);
                     }
 #pragma unroll
                     for (int j = 0; j < 32; ++j) {
@@ -435,7 +479,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                         const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u[j]));
                         g[j] = pack_bf16(x.x * sigmoid_fast(x.x) * y.x, x.y * sigmoid_fast(x.y) * y.y);
                     }
-                    wide_put_bf16<1>(out, p.ldc, g, col0, w.n_valid, rows, stage, lane);
+                    wide_put_bf16<1>(out, g, col0);
                 }
                 continue;
             }
@@ -446,10 +490,11 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 if (!(ok = ready(block))) break;
                 wide_take_bf16<4>(t_row + block * kBlockN, p.alpha, zero, v);
                 release(block);
-                wide_put_bf16<2>(out, p.ldc, v, block * 256 + half * 128, w.n_valid, rows, stage, lane);
+                wide_put_bf16<2>(out, v, block * 256 + half * 128);
             }
             if (!ok) break;
         }
+        if (lane == 0) tma_store_wait<0>();              // every block handed to TMA has been written
     }
 
     // ---------------- teardown ----------------

@@ -178,3 +178,19 @@ def test_every_product_on_the_pair_kernel_in_a_fresh_process():
     r = subprocess.run([sys.executable, "-m", "pytest", "tests/test_gemm_gpu.py", "tests/test_moe_gpu.py", "-q", "-m", "gpu", "-x",
                         "-k", "not fresh_process"], cwd=root, env=env, capture_output=True, text=True, timeout=900)
     assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("m,n", [(4096, 4096), (4090, 4092), (4096, 4000)])
+def test_accumulate_keeps_subnormals_and_neighbours(m, n):
+    """Whole 32-row blocks are added by TMA, ragged ones by the lanes; a zero product changes no bit of either, and nothing
+    outside the output's columns is touched."""
+    from halo_b200.ops.gemm import matmul
+
+    a = torch.zeros(m, 256, device="cuda", dtype=torch.bfloat16)
+    b = torch.zeros(n, 256, device="cuda", dtype=torch.bfloat16)
+    buf = torch.full((m, n + 64), 1e-40, device="cuda")
+    buf[:, 1::2] = -3e-41
+    buf[:, 2::64] = float("inf")
+    before = buf.clone()
+    matmul(a, b, out=buf[:, :n], accumulate=True)
+    assert torch.equal(buf.view(torch.int32), before.view(torch.int32))
