@@ -102,9 +102,10 @@ def stream_ptr(device: torch.device | None = None) -> c_void_p:
 
 def plain_inference() -> bool:
     """True where an operation may call its kernels without its autograd node: gradients are off and neither forward-mode
-    differentiation nor a functorch transform (vmap, grad, jvp) is active, so the node would record and pass on nothing."""
+    differentiation nor a functorch transform (vmap, grad, jvp) is active, so the node would record and pass on nothing.
+    Not while ``torch.jit.trace`` runs: it records the node as a call, but cannot see what a kernel writes through a pointer."""
     return (not torch.is_grad_enabled() and torch.autograd.forward_ad._current_level < 0
-            and torch._C._functorch.peek_interpreter_stack() is None)
+            and torch._C._functorch.peek_interpreter_stack() is None and not torch._C._is_tracing())
 
 
 def check(rc: int, what: str) -> None:
