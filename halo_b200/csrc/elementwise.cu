@@ -342,7 +342,9 @@ qknorm_rope_fwd_kernel(const __nv_bfloat16* __restrict__ qkv, const __nv_bfloat1
     const int pair0 = (int)(wid % splits) * kRopePairs;
     long long place = -1;        // this token's first cached element
     if (CACHE) {
-        const long long r = cache.rows[t], c = cache.cols[t];
+        long long r = cache.rows[t], c = cache.cols[t];
+        if (r < 0) r += cache.batch;                        // counted from the end, as index expressions do
+        if (c < 0) c += cache.max_len;
         if (r >= 0 && r < cache.batch && c >= 0 && c < cache.max_len) place = (r * cache.max_len + c) * Hkv * 128 + l16 * 8;
         else if (lane == 0 && cache.status) atomicCAS(cache.status, kStatusOk, kStatusBounds);
     }

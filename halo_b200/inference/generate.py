@@ -106,24 +106,32 @@ class KVCache:
 
     def rotate_and_write(self, qkv, attn, table, keep_keys: bool):
         """q / k norm, rotary embedding and the cache write of this layer in one kernel, or None where it does not apply (then
-        :func:`qk_norm_rope` and :meth:`write` do). Returns ``(q, k or None, layer index)``."""
+        :func:`qk_norm_rope` and :meth:`write` do: gradients or a transform, other types and widths, and index tensors that the
+        kernel cannot read element by element - on the host, or broadcast over the tokens). Returns ``(q, k or None, layer
+        index)``. Negative positions count from the end, as in an index expression; a position outside the cache is skipped
+        and recorded in the status word (:func:`halo_b200.ops._lib.raise_on_status`)."""
+        from halo_b200.ops import _lib
+
         cfg = attn.cfg
         Hq, Hkv, D = cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim
         wq, wk = attn.q_norm, attn.k_norm
-        if (not qkv.is_cuda or D != 128 or qkv.dtype != torch.bfloat16 or self.k.dtype != torch.bfloat16 or 2 * table.shape[1] != D
-                or tuple(self.k.shape[-2:]) != (Hkv, D) or qkv.shape[1] != (Hq + 2 * Hkv) * D or self._rows.dtype != torch.long
-                or self._cols.dtype != torch.long or (cfg.use_qk_norm and (wq is None or wq.numel() != D))
-                or (torch.is_grad_enabled() and qkv.requires_grad) or qkv.shape[0] == 0):
+        T, dev, gpu = qkv.shape[0], qkv.device, qkv.get_device()
+        rows, cols = self._rows, self._cols
+        if (not qkv.is_cuda or D != 128 or qkv.dtype != torch.bfloat16 or T == 0 or qkv.shape[1] != (Hq + 2 * Hkv) * D
+                or self.k.dtype != torch.bfloat16 or self.v.dtype != torch.bfloat16 or self.k.shape[-2:] != (Hkv, D)
+                or self.v.shape != self.k.shape or not self.k.is_contiguous() or not self.v.is_contiguous()
+                or rows.dtype != torch.long or cols.dtype != torch.long or rows.shape != (T,) or cols.shape != (T,)
+                or table.dtype != torch.float32 or table.shape != (T, D // 2, 2)
+                or any(t.get_device() != gpu for t in (self.k, self.v, rows, cols, table))
+                or (cfg.use_qk_norm and (wq is None or wq.numel() != D)) or not _lib.untransformed()
+                or (torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (qkv, wq, wk)))):
             return None
-        from halo_b200.ops import _lib
-
         li = self._layer
         self._layer += 1
-        qkv = qkv.contiguous()
-        T, dev = qkv.shape[0], qkv.device
+        qkv, table = qkv.contiguous(), table.contiguous()
         q = torch.empty((T, Hq * D), dtype=torch.bfloat16, device=dev)
         k = torch.empty((T, Hkv * D), dtype=torch.bfloat16, device=dev) if keep_keys else None
-        rows, cols = self._rows.contiguous(), self._cols.contiguous()
+        rows, cols = rows.contiguous(), cols.contiguous()
         rc = _lib.lib().halo_qknorm_rope_cache(
             _lib.ptr(qkv), _lib.ptr(wq), _lib.ptr(wk), _lib.ptr(table), _lib.ptr(q), _lib.ptr(k), _lib.ptr(self.k[li]),
             _lib.ptr(self.v[li]), _lib.ptr(rows), _lib.ptr(cols), _lib.c_ll(self.k.shape[1]), _lib.c_ll(self.k.shape[2]),

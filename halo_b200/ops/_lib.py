@@ -100,12 +100,16 @@ def stream_ptr(device: torch.device | None = None) -> c_void_p:
     return c_void_p(torch._C._cuda_getCurrentRawStream(index))
 
 
+def untransformed() -> bool:
+    """Nothing but reverse mode can be watching: no forward-mode differentiation, no functorch transform (vmap, grad, jvp), and no
+    ``torch.jit.trace``, which records an autograd node as a call but cannot see what a kernel writes through a pointer."""
+    return (torch.autograd.forward_ad._current_level < 0 and torch._C._functorch.peek_interpreter_stack() is None
+            and not torch._C._is_tracing())
+
+
 def plain_inference() -> bool:
-    """True where an operation may call its kernels without its autograd node: gradients are off and neither forward-mode
-    differentiation nor a functorch transform (vmap, grad, jvp) is active, so the node would record and pass on nothing.
-    Not while ``torch.jit.trace`` runs: it records the node as a call, but cannot see what a kernel writes through a pointer."""
-    return (not torch.is_grad_enabled() and torch.autograd.forward_ad._current_level < 0
-            and torch._C._functorch.peek_interpreter_stack() is None and not torch._C._is_tracing())
+    """True where an operation may call its kernels without its autograd node: the node would record and pass on nothing."""
+    return not torch.is_grad_enabled() and untransformed()
 
 
 def check(rc: int, what: str) -> None:

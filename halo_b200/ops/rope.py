@@ -185,4 +185,6 @@ def qk_norm_rope(qkv, wq, wk, table, n_heads, n_kv_heads, eps=1e-6, use_norm=Tru
     whole_width_norm = use_norm and wq is not None and wq.numel() != D
     if not qkv.is_cuda or D != HEAD_DIM or qkv.dtype != torch.bfloat16 or 2 * table.shape[1] != D or whole_width_norm:
         return qk_norm_rope_reference(qkv, wq, wk, table, n_heads, n_kv_heads, eps, use_norm)
+    if table.shape[0] < qkv.shape[0]:       # the kernel reads one row of angles per token
+        raise ValueError(f"the rotary table holds {table.shape[0]} positions for {qkv.shape[0]} tokens")
     return _QKNormRope.apply(qkv.contiguous(), wq, wk, table, n_heads, n_kv_heads, eps, use_norm)

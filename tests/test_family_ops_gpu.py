@@ -349,3 +349,44 @@ def test_family_on_gpu_follows_its_fp32_cpu_twin(family):
         norms.append(float(torch.sqrt(sum(g.float().pow(2).sum() for g in grads))))
     assert abs(losses[0] - losses[1]) <= 3e-2 * abs(losses[0]), (family, losses)
     assert abs(norms[0] - norms[1]) <= 0.15 * norms[0], (family, norms)
+
+
+@pytest.mark.parametrize("form", ["device", "host", "negative", "one sequence", "wrong length"])
+def test_cached_attention_takes_the_positions_an_index_expression_takes(form):
+    """Cache and output of a prefill against the same prefill through the separate rotation and scatter, bit for bit."""
+    from types import SimpleNamespace
+
+    from halo_b200.inference.generate import KVCache, cached_attention
+    from halo_b200.ops import _lib
+    from halo_b200.ops import attention as attn_ops
+    from halo_b200.ops.rope import qk_norm_rope, rope_table
+
+    torch.manual_seed(0)
+    T, heads, kv_heads, S = 33, 8, 2, 40
+    cfg = SimpleNamespace(num_attention_heads=heads, num_key_value_heads=kv_heads, head_dim=128, rms_norm_eps=1e-6, use_qk_norm=False)
+    qkv = torch.randn(T, (heads + 2 * kv_heads) * 128, device="cuda").bfloat16()
+    table = rope_table(torch.arange(T, device="cuda"), 128, 1e6)
+    plan = attn_ops.build_plan([0, T], device="cuda")
+    attn = SimpleNamespace(cfg=cfg, q_norm=None, k_norm=None, window=0, sinks=None, scale=None, softcap=0.0, _qkv=lambda h: h,
+                           _out=lambda o: o, rope_of=lambda ctx: table)
+    rows, cols = torch.zeros(T, dtype=torch.long, device="cuda") + 1, torch.arange(T, device="cuda")
+    given = {"device": (rows, cols), "host": (rows.cpu(), cols.cpu()), "negative": (rows - 3, cols - S),
+             "one sequence": (rows[:1], cols), "wrong length": (rows[:7], cols)}[form]
+    cache = KVCache(1, 3, S, kv_heads, 128, torch.bfloat16, "cuda")
+    cache.begin_prefill(*given, torch.tensor([T], device="cuda"))
+    ctx = SimpleNamespace(kv_cache=cache, plan=plan)
+    with torch.no_grad():
+        if form == "wrong length":
+            with pytest.raises((RuntimeError, IndexError)):
+                cached_attention(attn, qkv, ctx)
+            with pytest.raises(ValueError):
+                qk_norm_rope(qkv, None, None, table[:5], heads, kv_heads, 1e-6, False)
+            return
+        got = cached_attention(attn, qkv, ctx)
+        q, k = qk_norm_rope(qkv, None, None, table, heads, kv_heads, 1e-6, False)
+        v = qkv[:, (heads + kv_heads) * 128:]
+        want = attn_ops.flash_attention(q, k, v, plan, heads, kv_heads)
+    keys, values = torch.zeros_like(cache.k[0]), torch.zeros_like(cache.v[0])
+    keys[rows, cols] = k.view(T, kv_heads, 128)
+    values[rows, cols] = v.reshape(T, kv_heads, 128)
+    assert torch.equal(got, want) and torch.equal(cache.k[0], keys) and torch.equal(cache.v[0], values) and _lib.read_status() == 0

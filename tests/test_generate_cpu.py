@@ -242,3 +242,61 @@ def test_generation_callbacks(tmp_path):
     assert any("phase/whole" in rec for rec in trainer.log_history)
     with pytest.raises(MtpGateFailed, match="rejected"):
         run(0.0 + 1e-12, MtpAcceptanceGate(train, min_gain=0.2))     # nothing learned: the gate fails the run
+
+
+class _OnDevice(torch.Tensor):
+    """A host tensor that says it lives on the GPU the other tensors of the test live on."""
+
+    is_cuda = True
+
+    def get_device(self):
+        return 0
+
+
+def test_fused_cache_write_takes_only_what_the_kernel_can_read(monkeypatch):
+    """The kernel behind ``rotate_and_write`` reads one row, one position and one row of angles per token through raw
+    pointers. Index tensors on the host, broadcast ones, short ones and short tables are left to the indexed write."""
+    from types import SimpleNamespace
+
+    from halo_b200.inference.generate import KVCache
+    from halo_b200.ops import _lib
+
+    T, Hq, Hkv = 5, 4, 2
+    calls = []
+
+    class Library:
+        def __getattr__(self, name):
+            return lambda *a: calls.append(name) or 0
+
+    monkeypatch.setattr(_lib, "lib", Library)
+    monkeypatch.setattr(_lib, "status_word", lambda device: None)
+    monkeypatch.setattr(_lib, "stream_ptr", lambda device=None: None)
+    cfg = SimpleNamespace(num_attention_heads=Hq, num_key_value_heads=Hkv, head_dim=128, rms_norm_eps=1e-6, use_qk_norm=False)
+    attn = SimpleNamespace(cfg=cfg, q_norm=None, k_norm=None)
+
+    def on_device(t):
+        return t.as_subclass(_OnDevice)
+
+    qkv = on_device(torch.zeros(T, (Hq + 2 * Hkv) * 128, dtype=torch.bfloat16))
+    table = on_device(torch.zeros(T, 64, 2))
+    index = on_device(torch.arange(T))
+
+    def route(rows=index, cols=index, angles=table, x=qkv):
+        cache = KVCache(1, 8, 16, Hkv, 128, torch.bfloat16, "cpu")
+        cache.k, cache.v = on_device(cache.k), on_device(cache.v)
+        cache.begin_prefill(rows, cols, None)
+        return cache.rotate_and_write(x, attn, angles, keep_keys=True) is not None
+
+    assert route() and calls == ["halo_qknorm_rope_cache"]
+    assert not route(rows=torch.arange(T)) and not route(cols=torch.arange(T))
+    assert not route(rows=index[:1]) and not route(cols=index[:4]) and not route(cols=index[None])
+    assert not route(rows=on_device(torch.arange(T + 1)))
+    assert not route(cols=on_device(torch.arange(T, dtype=torch.int32)))
+    assert not route(angles=table[:1]) and not route(angles=torch.zeros(T, 64, 2)) and not route(angles=on_device(torch.zeros(T, 64, 2).double()))
+    tracked = on_device(torch.zeros_like(qkv)).requires_grad_()
+    assert not route(x=tracked)
+    with torch.no_grad():
+        assert route(x=tracked)
+        with torch.autograd.forward_ad.dual_level():
+            assert not route()
+    assert calls == ["halo_qknorm_rope_cache"] * 2
