@@ -55,7 +55,12 @@ def _ce_inplace(logits, labels, grad_scale, row_scale, ignore_index):
 
 
 def _scaled_bf16(x, g):
-    """``x`` (fp32 sums or bf16) rounded to bf16 and multiplied by the device scalar ``g``, in one pass."""
+    """``x`` (fp32 sums or bf16) rounded to bf16 and multiplied by the device scalar ``g``, in one pass. As tensor operations, with
+    the same roundings, where somebody differentiates with respect to ``g`` (``create_graph``) or batches over it
+    (``is_grads_batched``, functorch), and for what a saved-tensor hook returned that the kernel does not read."""
+    if (torch.is_grad_enabled() or not _lib.untransformed() or torch._C._functorch.is_legacy_batchedtensor(g) or not x.is_cuda
+            or x.dtype not in (torch.float32, torch.bfloat16) or not x.is_contiguous() or x.data_ptr() % 16):
+        return x.to(torch.bfloat16) * g.to(torch.bfloat16)
     out = torch.empty(x.shape, dtype=torch.bfloat16, device=x.device)
     rc = _lib.lib().halo_scale_to_bf16(_lib.ptr(x), _lib.c_int(1 if x.dtype == torch.float32 else 0),
                                        _lib.ptr(g.reshape(1).to(torch.float32)), _lib.ptr(out), _lib.c_ll(x.numel()),

@@ -77,3 +77,40 @@ def test_head_loss_edges_and_upstream_scale(T, V, chunk):
     lp = torch.log_softmax(z.detach(), -1)
     want = torch.where(labels == -100, 0.0, lp.gather(-1, labels.clamp_min(0)[:, None])[:, 0])
     assert (logp - want).abs().max() <= 2.0 ** -8 * 5 and (ent + (lp.exp() * lp).sum(-1)).abs().max() <= 2.0 ** -8 * 5
+
+
+@pytest.mark.filterwarnings("ignore::UserWarning")
+@pytest.mark.parametrize("mode", ["create_graph", "batched", "hooks"])
+def test_head_loss_gradients_by_the_uncommon_routes(mode):
+    """A derivative with respect to the upstream scalar, a batch of upstream scalars, and saved gradients that a hook hands
+    back in another layout: bit for bit what the plain backward gives for the same scalar."""
+    from halo_b200.ops.cross_entropy import fused_linear_cross_entropy
+
+    torch.manual_seed(0)
+    T, H, V = 70, 128, 520
+    h = torch.randn(T, H, device="cuda").bfloat16().requires_grad_()
+    w = (torch.randn(V, H, device="cuda") * H ** -0.5).bfloat16().requires_grad_()
+    labels = torch.randint(0, V, (T,), device="cuda")
+
+    def loss():
+        return fused_linear_cross_entropy(h, w, labels)
+
+    one, three = (torch.autograd.grad(loss(), [h, w], torch.tensor(g, device="cuda")) for g in (1.0, 3.0))
+    if mode == "create_graph":
+        g = torch.tensor(3.0, device="cuda", requires_grad=True)
+        got = torch.autograd.grad(loss(), [h, w], g, create_graph=True)
+        assert all(torch.equal(a, b) for a, b in zip(got, three))
+        for grad, unit in zip(got, one):
+            along = torch.randn_like(unit)
+            slope, = torch.autograd.grad(grad, g, along, retain_graph=True)
+            want = (unit.double() * along.double()).sum()
+            # the products are rounded to bf16 and summed in fp32
+            assert abs(slope - want) <= 2.0 ** -8 * (unit.double() * along.double()).abs().sum()
+    elif mode == "batched":
+        got = torch.autograd.grad(loss(), [h, w], torch.tensor([1.0, 3.0], device="cuda"), is_grads_batched=True)
+        for both, a, b in zip(got, one, three):
+            assert torch.equal(both[0], a) and torch.equal(both[1], b)
+    else:
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t.t().contiguous().t() if t.dim() == 2 else t):
+            got = torch.autograd.grad(loss(), [h, w], torch.tensor(3.0, device="cuda"))
+        assert all(torch.equal(a, b) for a, b in zip(got, three))
