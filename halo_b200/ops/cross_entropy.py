@@ -54,6 +54,15 @@ def _ce_inplace(logits, labels, grad_scale, row_scale, ignore_index):
     return loss, lse
 
 
+def _round_and_scale(x, g=None):
+    out = torch.empty(x.shape, dtype=torch.bfloat16, device=x.device)
+    g32 = g.reshape(1).to(torch.float32) if g is not None else None
+    rc = _lib.lib().halo_scale_to_bf16(_lib.ptr(x), _lib.c_int(1 if x.dtype == torch.float32 else 0), _lib.ptr(g32), _lib.ptr(out),
+                                       _lib.c_ll(x.numel()), _lib.stream_ptr(x.device))
+    _lib.check(rc, "halo_scale_to_bf16")
+    return out
+
+
 def _scaled_bf16(x, g):
     """``x`` (fp32 sums or bf16) rounded to bf16 and multiplied by the device scalar ``g``, in one pass. As tensor operations, with
     the same roundings, where somebody differentiates with respect to ``g`` (``create_graph``) or batches over it
@@ -61,12 +70,7 @@ def _scaled_bf16(x, g):
     if (torch.is_grad_enabled() or not _lib.untransformed() or torch._C._functorch.is_legacy_batchedtensor(g) or not x.is_cuda
             or x.dtype not in (torch.float32, torch.bfloat16) or not x.is_contiguous() or x.data_ptr() % 16):
         return x.to(torch.bfloat16) * g.to(torch.bfloat16)
-    out = torch.empty(x.shape, dtype=torch.bfloat16, device=x.device)
-    rc = _lib.lib().halo_scale_to_bf16(_lib.ptr(x), _lib.c_int(1 if x.dtype == torch.float32 else 0),
-                                       _lib.ptr(g.reshape(1).to(torch.float32)), _lib.ptr(out), _lib.c_ll(x.numel()),
-                                       _lib.stream_ptr(x.device))
-    _lib.check(rc, "halo_scale_to_bf16")
-    return out
+    return _round_and_scale(x, g)
 
 
 def _head_grad_buffer(weight, rows):
@@ -99,7 +103,8 @@ class _FusedLinearCE(torch.autograd.Function):
                 matmul(logits, weight, b_t=False, out=dh[s:e])
             if need_dw:
                 matmul(logits, hc, a_t=True, b_t=False, out=dw32, accumulate=s > 0)
-        ctx.save_for_backward(dh, dw32)
+        # a pending loss holds the head's gradient in bf16, half of its sums: several may be pending at once
+        ctx.save_for_backward(dh, _round_and_scale(dw32) if need_dw else None)
         return loss_sum * grad_scale
 
     @staticmethod

@@ -114,3 +114,21 @@ def test_head_loss_gradients_by_the_uncommon_routes(mode):
         with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t.t().contiguous().t() if t.dim() == 2 else t):
             got = torch.autograd.grad(loss(), [h, w], torch.tensor(3.0, device="cuda"))
         assert all(torch.equal(a, b) for a, b in zip(got, three))
+
+
+def test_a_pending_loss_holds_its_head_gradient_once_in_bf16():
+    """What stays allocated between forward and backward: both gradients in bf16 and a few scalars, not the fp32 sums."""
+    from halo_b200.ops.cross_entropy import fused_linear_cross_entropy
+
+    T, H, V = 64, 512, 32768
+    h = torch.randn(T, H, device="cuda").bfloat16().requires_grad_()
+    w = torch.randn(V, H, device="cuda").bfloat16().requires_grad_()
+    labels = torch.randint(0, V, (T,), device="cuda")
+    fused_linear_cross_entropy(h, w, labels)            # workspaces of the first call
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    loss = fused_linear_cross_entropy(h, w, labels)
+    held = torch.cuda.memory_allocated() - before
+    assert 2 * V * H <= held <= 2 * (V + T) * H + (1 << 20)
+    loss.backward()
+    assert w.grad.dtype == torch.bfloat16
