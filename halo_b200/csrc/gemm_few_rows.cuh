@@ -32,6 +32,21 @@ constexpr int kFewThreads = 192;
 constexpr int kFewMaxStages = 6;
 constexpr int kFewWBytes = 128 * kBlockK * 2;      // weight tile of one stage: 128 rows x 64
 
+// The ring for tiles of m_pad columns: two CTAs an SM up to 128 columns, one above. Once all products are done it holds the
+// [m_pad][128] fp32 partial sums.
+__host__ __device__ constexpr int few_stage_bytes(int m_pad) { return kFewWBytes + m_pad * kBlockK * 2; }
+__host__ __device__ constexpr int few_stages(int m_pad) {
+    const int n = (m_pad <= 128 ? 110 : 220) * 1024 / few_stage_bytes(m_pad);
+    return n < kFewMaxStages ? n : kFewMaxStages;
+}
+__host__ __device__ constexpr int few_smem_bytes(int m_pad) { return few_stages(m_pad) * few_stage_bytes(m_pad) + 1024; }     // + alignment
+__host__ __device__ constexpr bool few_sums_fit(int m_pad) { return m_pad * 128 * 4 <= few_stages(m_pad) * few_stage_bytes(m_pad); }
+static_assert(few_sums_fit(16) && few_sums_fit(32) && few_sums_fit(64) && few_sums_fit(128) && few_sums_fit(256),
+              "the partial sums fit over the ring");
+constexpr int kFewMaxSmemBytes = few_smem_bytes(256);
+static_assert(few_smem_bytes(16) <= kFewMaxSmemBytes && few_smem_bytes(32) <= kFewMaxSmemBytes &&
+              few_smem_bytes(64) <= kFewMaxSmemBytes && few_smem_bytes(128) <= kFewMaxSmemBytes, "the widest tile needs the most");
+
 struct FewParams {
     void* C;
     void* aux;           // SwiGLU: optional [M, 2F] pre-activations
@@ -64,7 +79,7 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t rank = cluster_cta_rank();
     const int tile = blockIdx.x / p.parts;
-    const int stage_bytes = kFewWBytes + p.m_pad * kBlockK * 2;
+    const int stage_bytes = few_stage_bytes(p.m_pad);
     const int tmem_cols = p.m_pad < 32 ? 32 : p.m_pad;
 
     if (threadIdx.x == 0) {

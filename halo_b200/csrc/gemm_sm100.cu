@@ -433,13 +433,11 @@ static int launch_few_rows(const void* X, const void* W, long long ldx, long lon
     if (rc) return rc;
     rc = make_tmap_bf16(&tw, W, p.N, p.K, ldw, p.swiglu_f ? 64 : 128);
     if (rc) return rc * 10;
-    // the ring also holds the [m_pad][128] fp32 partial sums: m_pad * 512 bytes, less than two stages
-    const int stage_bytes = kFewWBytes + p.m_pad * kBlockK * 2;
-    p.stages = (p.m_pad <= 128 ? 110 : 220) * 1024 / stage_bytes;
-    if (p.stages > kFewMaxStages) p.stages = kFewMaxStages;
-    const int smem = p.stages * stage_bytes + 1024;
-    // set for the current device at every launch (no state is kept here)
-    if (cudaFuncSetAttribute(gemm_few_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -10;
+    p.stages = few_stages(p.m_pad);
+    const int smem = few_smem_bytes(p.m_pad);
+    // Set for the current device at every launch, and always to what the widest tile needs: the attribute belongs to the function,
+    // and another thread's call for another tile may come between this one's attribute and its launch.
+    if (cudaFuncSetAttribute(gemm_few_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewMaxSmemBytes) != cudaSuccess) return -10;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(n_tiles * p.parts), 1, 1);
     cfg.blockDim = dim3(kFewThreads, 1, 1);
@@ -452,7 +450,9 @@ static int launch_few_rows(const void* X, const void* W, long long ldx, long lon
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, gemm_few_rows_kernel, tw, tx, p) == cudaSuccess ? 0 : -11;
+    if (cudaLaunchKernelEx(&cfg, gemm_few_rows_kernel, tw, tx, p) == cudaSuccess) return 0;
+    cudaGetLastError();                 // reported here, not at a later launch's check
+    return -11;
 }
 
 template <bool A_MN, bool B_MN>
@@ -476,7 +476,9 @@ static int launch_wide_t(const CUtensorMap& ta, const CUtensorMap& tb, const CUt
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, gemm_wide_kernel<A_MN, B_MN>, ta, tb, tc, tx, p) == cudaSuccess ? 0 : -11;
+    if (cudaLaunchKernelEx(&cfg, gemm_wide_kernel<A_MN, B_MN>, ta, tb, tc, tx, p) == cudaSuccess) return 0;
+    cudaGetLastError();                 // reported here, not at a later launch's check
+    return -11;
 }
 
 static int launch_wide(int a_mn, int b_mn, const CUtensorMap& ta, const CUtensorMap& tb, GemmParams p, int n_pairs, cudaStream_t s) {

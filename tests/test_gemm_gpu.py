@@ -194,3 +194,39 @@ def test_accumulate_keeps_subnormals_and_neighbours(m, n):
     before = buf.clone()
     matmul(a, b, out=buf[:, :n], accumulate=True)
     assert torch.equal(buf.view(torch.int32), before.view(torch.int32))
+
+
+def test_few_rows_from_two_threads():
+    """Two threads on streams of their own, one with the smallest tile's ring and one with the largest: a launch gets the
+    shared memory it asks for whatever the other thread's call sets in between."""
+    import threading
+
+    from halo_b200.ops import _lib
+    from halo_b200.ops.gemm import matmul
+
+    torch.manual_seed(0)
+    w = torch.randn(512, 4096, device="cuda").bfloat16()
+    torch.cuda.synchronize()
+    failures = []
+
+    def work(rows):
+        try:
+            x = torch.ones(rows, 4096, device="cuda").bfloat16()
+            with torch.cuda.stream(torch.cuda.Stream()):
+                torch.cuda.current_stream().wait_stream(torch.cuda.default_stream())
+                out = torch.empty(rows, 512, device="cuda", dtype=torch.bfloat16)
+                for _ in range(4000):
+                    matmul(x, w, out=out)
+                torch.cuda.current_stream().synchronize()
+            want = w.double().sum(1)
+            assert ((out - want).abs() <= 2.0 ** -8 * want.abs() + 0.05).all()
+        except BaseException as exc:
+            failures.append(exc)
+
+    threads = [threading.Thread(target=work, args=(rows,)) for rows in (16, 200)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures
+    assert _lib.read_status() == 0
