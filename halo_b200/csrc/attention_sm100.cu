@@ -241,7 +241,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         for (int i = 0; i < 128; ++i) acc[i] = 0.f;
         bool ok = true;
         for (int j = 0; j < w.n_kv; ++j) {
-            if (!mbar_wait(smem_u32(&bar_s_full), j & 1, &abort_flag, p.status)) { ok = false; break; }
+            if (!mbar_wait_warp(smem_u32(&bar_s_full), j & 1, &abort_flag, p.status)) { ok = false; break; }
             tc_fence_after();
             const bool diag = (j == w.n_kv - 1);
             float mx = m;
@@ -293,7 +293,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             fence_proxy_async_smem();
             tc_fence_before();
             mbar_arrive(smem_u32(&bar_p_ready));
-            if (!mbar_wait(smem_u32(&bar_o_full), j & 1, &abort_flag, p.status)) { ok = false; break; }
+            if (!mbar_wait_warp(smem_u32(&bar_o_full), j & 1, &abort_flag, p.status)) { ok = false; break; }
             tc_fence_after();
 #pragma unroll
             for (int cc = 0; cc < 128; cc += 32) {
@@ -548,8 +548,8 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                 s_delta[it & 1][threadIdx.x] = in ? p.delta[(long long)h * p.T + qa] : 0.f;
                 mbar_arrive(smem_u32(&bar_stats));
             }
-            if (!mbar_wait(smem_u32(&bar_stats), it & 1, &abort_flag, p.status)) { ok = false; break; }
-            if (!mbar_wait(smem_u32(&bar_s_full), it & 1, &abort_flag, p.status)) { ok = false; break; }
+            if (!mbar_wait_warp(smem_u32(&bar_stats), it & 1, &abort_flag, p.status)) { ok = false; break; }
+            if (!mbar_wait_warp(smem_u32(&bar_s_full), it & 1, &abort_flag, p.status)) { ok = false; break; }
             tc_fence_after();
             const bool need_mask = (qr < w.kv0 + 128);
             float pv[64];
@@ -601,9 +601,9 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             tc_fence_before();
             mbar_arrive(smem_u32(&bar_ds_ready));
             // P^T may be overwritten next iteration only after the dV product has read it
-            if (!mbar_wait(smem_u32(&bar_dv_done), it & 1, &abort_flag, p.status)) { ok = false; break; }
+            if (!mbar_wait_warp(smem_u32(&bar_dv_done), it & 1, &abort_flag, p.status)) { ok = false; break; }
         }
-        if (ok && mbar_wait(smem_u32(&bar_acc_done), 0, &abort_flag, p.status)) {
+        if (ok && mbar_wait_warp(smem_u32(&bar_acc_done), 0, &abort_flag, p.status)) {
             tc_fence_after();
             // tcgen05.ld is warp-collective: every lane issues the loads, only the stores are guarded
             const bool live = key_abs < w.q_end;
@@ -771,7 +771,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const float dl = in ? p.delta[(long long)head * p.T + q_abs] : 0.f;
         bool ok = true;
         for (int j = 0; j < w.n_kv; ++j) {
-            if (!mbar_wait(smem_u32(&bar_s_full), j & 1, &abort_flag, p.status)) { ok = false; break; }
+            if (!mbar_wait_warp(smem_u32(&bar_s_full), j & 1, &abort_flag, p.status)) { ok = false; break; }
             tc_fence_after();
             const int k0 = w.kv0 + j * 64;
             const bool need_mask = (k0 + 64 > w.q0);
@@ -790,7 +790,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                 }
             }
             // the previous dQ product must have finished reading dS before it is overwritten
-            if (j > 0 && !mbar_wait(smem_u32(&bar_dq_done), (j - 1) & 1, &abort_flag, p.status)) { ok = false; break; }
+            if (j > 0 && !mbar_wait_warp(smem_u32(&bar_dq_done), (j - 1) & 1, &abort_flag, p.status)) { ok = false; break; }
 #pragma unroll
             for (int q8 = 0; q8 < 8; ++q8) {
                 const uint32_t a = sDS + swz_off(row, q8 * 8);
@@ -803,7 +803,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             tc_fence_before();
             mbar_arrive(smem_u32(&bar_ds_ready));
         }
-        if (ok && mbar_wait(smem_u32(&bar_acc_done), 0, &abort_flag, p.status)) {
+        if (ok && mbar_wait_warp(smem_u32(&bar_acc_done), 0, &abort_flag, p.status)) {
             tc_fence_after();
             __nv_bfloat16* dq = reinterpret_cast<__nv_bfloat16*>(p.dQ) + q_abs * p.ld_dq + head * kHd;
 #pragma unroll 1
@@ -1070,7 +1070,7 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             if (!ok) continue;
             const float* lse_b = s_lse + b * 64 + c0;
             const float* delta_b = s_delta + b * 64 + c0;
-            if (!mbar_wait(bar(kSFull + b), (it >> 1) & 1, abort_flag, p.status)) { ok = false; continue; }
+            if (!mbar_wait_warp(bar(kSFull + b), (it >> 1) & 1, abort_flag, p.status)) { ok = false; continue; }
             tc_fence_after();
             uint32_t sr[16], dr[16];
             tmem_ld_32x16(tS, sr);
@@ -1108,7 +1108,7 @@ attn_bwd_dkdv2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         }
         // the accumulators: parts 0 and 1 store dK, 2 and 3 dV (each thread one row, 64 of its 128 columns)
         const int g = part >> 1, half = part & 1;
-        if (ok && mbar_wait(bar(kAccDone), 0, abort_flag, p.status)) {
+        if (ok && mbar_wait_warp(bar(kAccDone), 0, abort_flag, p.status)) {
             tc_fence_after();
             bool live = key_abs < w.q_end;
             long long ld = g == 0 ? p.ld_dk : p.ld_dv;
@@ -1297,7 +1297,7 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const float lse2 = in ? p.lse[(long long)head * p.T + q_local] * kLog2e : INFINITY;
         const float dl = in ? p.delta[(long long)head * p.T + q_local] : 0.f;
         // parts 0 and 1 move Q to tensor memory, 2 and 3 dO: a thread 64 columns (128 swizzled bytes) of its row
-        bool ok = mbar_wait(bar(kQ), 0, abort_flag, p.status);
+        bool ok = mbar_wait_warp(bar(kQ), 0, abort_flag, p.status);
         if (ok) {
             uint32_t a[32];
             const uint32_t src = (part < 2 ? sQ : sdO) + (part & 1) * 16384 + row * 128;
@@ -1314,7 +1314,7 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         for (int j = 0; ok && j < w.n_kv; ++j) {
             const int b = j & 1;
             const uint32_t tS = tm0 + 128 * b + lane_base + c0, tDP = tS + 64;
-            if (!mbar_wait(bar(kSFull + b), (j >> 1) & 1, abort_flag, p.status)) { ok = false; break; }
+            if (!mbar_wait_warp(bar(kSFull + b), (j >> 1) & 1, abort_flag, p.status)) { ok = false; break; }
             tc_fence_after();
             uint32_t sr[16], dr[16];
             tmem_ld_32x16(tS, sr);
@@ -1344,7 +1344,7 @@ attn_bwd_dq2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             warp_arrive(bar(kDsReady + b), lane);
         }
         // the accumulator: every thread stores 32 of its row's 128 columns
-        if (ok && mbar_wait(bar(kAccDone), 0, abort_flag, p.status)) {
+        if (ok && mbar_wait_warp(bar(kAccDone), 0, abort_flag, p.status)) {
             tc_fence_after();
             const int col = part * 32;
             __nv_bfloat16* dq = reinterpret_cast<__nv_bfloat16*>(p.dQ) + q_local * p.ld_dq + head * kHd + col;
@@ -1505,7 +1505,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         float m_ref = -INFINITY, l = 0.f;
         bool ok = true;
         for (int j = 0; j < w.n_kv; ++j) {
-            if (!mbar_wait(bar_s_full[j & 1], (j >> 1) & 1, abort_flag, p.status)) { ok = false; break; }
+            if (!mbar_wait_warp(bar_s_full[j & 1], (j >> 1) & 1, abort_flag, p.status)) { ok = false; break; }
             tc_fence_after();
             const uint32_t tSj = tS + (j & 1) * 64;
             const int k0 = w.kv0 + j * 64;
@@ -1529,7 +1529,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 }
             }
             // the previous P V product must be done before P is overwritten or O is rescaled
-            if (j > 0 && !mbar_wait(bar_o_full, (j - 1) & 1, abort_flag, p.status)) { ok = false; break; }
+            if (j > 0 && !mbar_wait_warp(bar_o_full, (j - 1) & 1, abort_flag, p.status)) { ok = false; break; }
             const bool grow = (mx - m_ref) * c > 8.f;   // also true on the first tile (m_ref = -inf)
             if (__any_sync(0xffffffffu, grow)) {
                 const float alpha = fast_exp2((m_ref - mx) * c);
@@ -1592,7 +1592,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_p_ready);
         }
-        if (ok && mbar_wait(bar_o_full, (w.n_kv - 1) & 1, abort_flag, p.status)) {
+        if (ok && mbar_wait_warp(bar_o_full, (w.n_kv - 1) & 1, abort_flag, p.status)) {
             tc_fence_after();
             const bool live = q_abs < w.q_end;
             l = add_sink(l, m_ref * p.scale, p.sinks, head);
@@ -1762,7 +1762,7 @@ attn_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         float m_ref = -INFINITY, l = 0.f;
         bool ok = true;
         for (int j = 0; j < w.n_kv; ++j) {
-            if (!mbar_wait(bar_s_full[j & 1], (j >> 1) & 1, abort_flag, p.status)) { ok = false; break; }
+            if (!mbar_wait_warp(bar_s_full[j & 1], (j >> 1) & 1, abort_flag, p.status)) { ok = false; break; }
             tc_fence_after();
             const uint32_t tSj = tS + (j & 1) * 64;
             const int k0 = w.kv0 + j * 64;
@@ -1801,7 +1801,7 @@ attn_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 if (j > 0) {
                     // O is rescaled: the previous P V product must be done. Otherwise its completion is waited for below, behind
                     // the exponentials (P goes over this tile's own scores, which that product does not read).
-                    if (!mbar_wait(bar_o_full, (j - 1) & 1, abort_flag, p.status)) { ok = false; break; }
+                    if (!mbar_wait_warp(bar_o_full, (j - 1) & 1, abort_flag, p.status)) { ok = false; break; }
                     product_done = true;
                     tc_fence_after();
 #pragma unroll 1
@@ -1848,12 +1848,12 @@ attn_fwd3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             l += rs;
             // every phase of the barrier is waited for in turn, and before this tile's product can complete the next one: a
             // parity would not tell two phases apart
-            if (!product_done && !mbar_wait(bar_o_full, (j - 1) & 1, abort_flag, p.status)) { ok = false; break; }
+            if (!product_done && !mbar_wait_warp(bar_o_full, (j - 1) & 1, abort_flag, p.status)) { ok = false; break; }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_p_ready);
         }
-        if (ok && mbar_wait(bar_o_full, (w.n_kv - 1) & 1, abort_flag, p.status)) {
+        if (ok && mbar_wait_warp(bar_o_full, (w.n_kv - 1) & 1, abort_flag, p.status)) {
             tc_fence_after();
             const bool live = q_abs < w.q_end;
             l = add_sink(l, m_ref * p.scale, p.sinks, head);

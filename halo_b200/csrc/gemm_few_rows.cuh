@@ -146,7 +146,7 @@ gemm_few_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
         // partial sums to shared memory, token-major: [m_pad][128] fp32 over the ring, which is dead once all MMAs are done
         const int quarter = warp & 3;
         float* part = reinterpret_cast<float*>(smem_raw + (base - smem_u32(smem_raw)));
-        if (mbar_wait(smem_u32(&bar_done), 0, &abort_flag, p.status)) {
+        if (mbar_wait_warp(smem_u32(&bar_done), 0, &abort_flag, p.status)) {
             tc_fence_after();
             const uint32_t t_row = tmem + (uint32_t(quarter * 32) << 16);
 #pragma unroll 1

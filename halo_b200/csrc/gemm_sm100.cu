@@ -153,8 +153,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         int acc = 0;
         uint32_t acc_phase = 0;
         GemmWork w;
-        for (int idx = blockIdx.x; fetch_work(p, idx, total, w) && !abort_flag; idx += gridDim.x) {
-            if (!mbar_wait(smem_u32(&bar_tfull[acc]), acc_phase, &abort_flag, p.status)) break;
+        for (int idx = blockIdx.x; fetch_work(p, idx, total, w) && !warp_aborted(&abort_flag); idx += gridDim.x) {
+            if (!mbar_wait_warp(smem_u32(&bar_tfull[acc]), acc_phase, &abort_flag, p.status)) break;
             tc_fence_after();
             const uint32_t t_row = tmem_base + acc * kBlockN + (uint32_t(quarter * 32) << 16);
             epilogue_tile(p, w, t_row, row_in_tile, epi_stage);

@@ -413,7 +413,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         uint32_t used[2] = {0, 0};
         GemmWork w, next;
         auto ready = [&](int block) -> bool {            // the block's products are complete
-            if (!mbar_wait(smem_u32(&bar_tfull[block]), used[block]++ & 1u, &abort_flag, p.status)) return false;
+            if (!mbar_wait_warp(smem_u32(&bar_tfull[block]), used[block]++ & 1u, &abort_flag, p.status)) return false;
             tc_fence_after();
             return true;
         };
@@ -423,7 +423,7 @@ gemm_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             if (lane == 0) mbar_arrive_remote(map_to_cta(smem_u32(&bar_tempty[block]), 0));
         };
         bool more = wide_fetch(p, first, total, next);
-        for (int idx = first + step; more && !abort_flag; idx += step) {
+        for (int idx = first + step; more && !warp_aborted(&abort_flag); idx += step) {
             w = next;
             more = wide_fetch(p, idx, total, next);
             const int rows = max(0, min(32, w.m_valid - int(rank) * 128 - row0));       // rows of this warp that exist

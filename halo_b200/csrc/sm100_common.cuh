@@ -99,9 +99,15 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
 }
 
-// The same for a whole converged warp, with one answer for all its lanes.
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status) {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status));
+// The same for a whole converged warp, with one answer for all its lanes: a lane that gave up alone would leave the others in
+// the next warp-wide instruction or barrier, which has no limit.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status,
+                                               uint64_t budget_ns = HALO_WAIT_BUDGET_NS) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, budget_ns));
+}
+// Whether a whole converged warp should stop: one answer for all its lanes.
+__device__ __forceinline__ bool warp_aborted(const volatile int* abort_flag) {
+    return __any_sync(0xffffffffu, *abort_flag != 0);
 }
 
 __device__ __forceinline__ void fence_proxy_async_smem() {

@@ -98,6 +98,29 @@ def test_device_code_rules():
             pytest.fail(f"{path}: an unbounded mbarrier spin near offset {m.start()}")
 
 
+def test_whole_warps_wait_and_leave_as_one():
+    """A wait that may give up answers each lane for itself. In a role that a whole warp walks - tensor-memory loads and
+    barriers that take every lane - lanes that disagree would wait for one another without a limit. So the per-lane wait
+    stands only under `lane == 0`, and a loop condition elsewhere does not read the abort flag lane by lane."""
+    hits = []
+    for path in sources(".cu", ".cuh"):
+        if path.endswith("sm100_common.cuh"):
+            continue
+        text = re.sub(r"//[^\n]*", lambda m: " " * len(m.group(0)), read(path))
+        for m in re.finditer(r"\bmbar_wait\(|\bfor \([^{}]*&& !abort_flag", text):
+            headers, start = [], 0
+            for i, ch in enumerate(text[:m.start()]):
+                if ch == "{":
+                    headers.append(text[start:i])
+                elif ch == "}" and headers:
+                    headers.pop()
+                if ch in "{};":
+                    start = i + 1
+            if not any("lane == 0" in h for h in headers):
+                hits.append(f"{path}:{text[:m.start()].count(chr(10)) + 1}: {m.group(0)[:60]}")
+    assert not hits, "\n".join(hits)
+
+
 # ---- bindings and entry points -------------------------------------------------------------------------------------
 def test_every_bound_entry_point_exists_in_the_sources():
     exported = set()
