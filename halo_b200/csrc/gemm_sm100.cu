@@ -408,15 +408,20 @@ static int dispatch_gemm(int a_mn, int b_mn, const CUtensorMap& ta, const CUtens
     return launch_gemm<true, false>(ta, tb, p, grid, s);
 }
 
-// Whether gemm_few_rows_kernel takes a product (both operands K-major, plain store or SwiGLU). The lines follow the table in
-// gemm_few_rows.cuh: up to 16 rows it always wins; above that the tokens' own tiles, which every CTA re-reads from L2, grow
-// with M while the large-tile kernels gain CTAs with N, so wide outputs stay there (`tiles_n`: their tiles along N). Above
-// 128 rows only one CTA fits an SM, which pays where the large tiles leave three quarters of the SMs idle.
+// Whether gemm_few_rows_kernel takes a product (both operands K-major, plain store or SwiGLU). Three things set the lines
+// (few-row kernel / the better large-tile kernel, us, weights cycled past L2):
+//  * It hands out the tokens one after the other when the products are done, which a short reduction does not cover. Up to 16
+//    rows it wins all the same, except by a microsecond for outputs of one tile; above that from K = 1024 on, above 64 rows from
+//    2048 (4096 columns: 17 rows K = 512 / 1024  7.5 / 8.3 against 7.8 / 11.7; 64 rows 11.4 / 10.1 against 7.9 / 11.6;
+//    128 rows K = 512 / 1024 / 2048  17.0 / 12.8 / 14.4 against 8.8 / 12.5 / 18.5).
+//  * The tokens' own tiles, which every CTA re-reads from L2, grow with M while the large tiles gain CTAs with N (`tiles_n`), so
+//    wide outputs stay there: 12,288 columns are for up to 64 rows and K >= 2048 (K = 1024 / 2048: 1.18 / 1.00 of their time).
+//  * Above 128 rows only one CTA fits an SM, which pays where the large tiles leave three quarters of the SMs idle.
 static bool few_rows_wins(int M, int N, int K, int tiles_n, bool glu) {
-    if (M <= 16) return true;
-    if (M <= 64) return tiles_n <= 48;
-    if (M <= 128) return tiles_n <= 32;
-    return M <= 256 && !glu && K >= 4096 && (N + 127) / 128 * 4 <= 148;
+    if (M <= 16) return glu || M <= 8 || K >= 1024 || N > 128;
+    if (M <= 64) return K >= 1024 && (tiles_n <= 32 || (tiles_n <= 48 && K >= 2048));
+    if (M <= 128) return K >= 2048 && tiles_n <= 32;
+    return M <= 256 && !glu && K >= 4096 && (N + 127) / 128 * 4 <= num_sms();
 }
 
 static int launch_few_rows(const void* X, const void* W, long long ldx, long long ldw, FewParams p, cudaStream_t stream) {
@@ -424,7 +429,7 @@ static int launch_few_rows(const void* X, const void* W, long long ldx, long lon
     while (p.m_pad < p.M) p.m_pad *= 2;
     const int n_tiles = p.swiglu_f ? (p.swiglu_f + 63) / 64 : (p.N + 127) / 128;
     const int kb = (p.K + kBlockK - 1) / kBlockK;
-    // cut the reduction while the clusters still fit the SMs at once and a part keeps at least 8 blocks of it
+    // cut the reduction while the clusters still fit the SMs at once and a part keeps at least 4 blocks of it
     const int slots = (p.m_pad <= 128 ? 2 : 1) * num_sms(), most = p.m_pad <= 128 ? 8 : 4;
     p.parts = 1;
     while (p.parts < most && n_tiles * p.parts * 2 <= slots && kb >= 8 * p.parts) p.parts *= 2;

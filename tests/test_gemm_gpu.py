@@ -52,7 +52,8 @@ def test_matmul_fp32_and_accumulate():
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 128, 64), (3, 136, 200), (16, 4096, 4096), (17, 1000, 776), (64, 2048, 12288), (65, 264, 8200),
-                                   (128, 8192, 512), (129, 4096, 4096), (256, 520, 4104), (257, 264, 4096)])
+                                   (128, 8192, 512), (129, 4096, 4096), (256, 520, 4104), (257, 264, 4096), (16, 128, 1016),
+                                   (16, 136, 1016), (17, 520, 1024), (33, 8200, 2048), (64, 520, 1016), (128, 1000, 2048), (100, 8200, 2056)])
 def test_few_rows(M, N, K):
     """Products with few rows at the edges of the dispatch (16, 64, 128 and 256 rows; one to eight cuts of the reduction,
     ragged N and K): bf16, fp32 and SwiGLU stores into strided outputs against 64-bit sums. fp32 sums of K products of
