@@ -568,21 +568,32 @@ int halo_gemm_bf16(const void* A, const void* B, void* C, void* aux, int M, int 
         p.tiles_n = (N + kBlockN - 1) / kBlockN;
     }
     p.list = nullptr; p.list_count = nullptr; p.status = status;
-    // Which kernel: the one whose waves of tiles take fewer cycles per 64-wide block of the reduction. A 256 x 512 tile keeps a
+    // Which kernel. First the one whose waves of tiles take fewer cycles per 64-wide block of the reduction: a 256 x 512 tile keeps a
     // pair of SMs 1,024 cycles at the rate the wide kernel reaches (0.92 of the tensor pipe, measured), a 128 x 256 tile one SM
-    // 512 cycles at 0.78. The wide kernel takes everything with more than a wave of tiles; the single-CTA kernel is left with
-    // products of few rows, where a 256-row tile would be padding, and with HALO_GEMM_PAIR=0.
-    if (g_use_pair && K > 0 && epi != kEpiClampedGlu) {
+    // 512 cycles at 0.78. That says nothing about what surrounds the products; where it decides (wide / single, us):
+    //  * One wave of single tiles is latency, and the pair's launch and epilogue are longer: bf16 4096 x 64 x 64  8 / 6, 600 x 2048 x
+    //    512  10 / 9. The wide kernel is quicker at fp32 (4096 x 768 x 256  10 / 15) unless half the tile is padding (4096 x 128 x
+    //    512  10 / 9).
+    //  * SwiGLU without the pre-activations: little is stored, and the single kernel's second accumulator hides it, which pays for
+    //    reductions from 512 to 2048 (8192 x 2 x 6144, K = 256 / 512 / 2048 / 4096  86 / 117 / 325 / 595 against 94 / 104 / 295 / 639).
+    //  * bf16 +=: the lanes read and write C themselves, and the wide kernel has no second tile to do it under
+    //    (16384 x 12288 x 4096  1,746 / 1,312; 4096 x 24576 x 8192  1,168 / 1,354).
+    // Over 4,860 shapes timed on both sides (all stores but fp32 +=, which the wide kernel is never slower at) the chosen kernel is
+    // within 0.7 % of the better one on average; by the waves alone 3.3 %.
+    const long long single_tiles = (long long)p.tiles_m * p.tiles_n;
+    const bool stores = epi == kEpiStoreBf16 || epi == kEpiStoreF32;
+    const bool stay = (stores && single_tiles <= num_sms() && (epi == kEpiStoreBf16 || N <= 128)) ||
+                      (glu && !aux && K > 256 && K <= 2048) || (epi == kEpiAccumBf16 && K <= 4096);
+    if (g_use_pair && K > 0 && epi != kEpiClampedGlu && (g_use_pair == 2 || !stay)) {
         GemmParams wide = p;
         const int pairs = num_sms() / 2, n_pairs = plan_wide(wide, pairs);
         const long long whole = (wide.wide_full + pairs - 1) / pairs, halves = wide.wide_items > wide.wide_full ? 1 : 0;
         const double wide_cost = (1024.0 * whole + 512.0 * halves) / 0.92;
-        const double single_cost = 512.0 * (((long long)p.tiles_m * p.tiles_n + num_sms() - 1) / num_sms()) / 0.78;
+        const double single_cost = 512.0 * ((single_tiles + num_sms() - 1) / num_sms()) / 0.78;
         if (g_use_pair == 2 || wide_cost <= single_cost)
             return launch_wide(a_mn_major, b_mn_major, ta, tb, wide, n_pairs, (cudaStream_t)stream);
     }
-    long long tiles = (long long)p.tiles_m * p.tiles_n;
-    int grid = (int)(tiles < num_sms() ? tiles : num_sms());
+    int grid = (int)(single_tiles < num_sms() ? single_tiles : num_sms());
     return dispatch_gemm(a_mn_major, b_mn_major, ta, tb, p, grid, (cudaStream_t)stream);
 }
 

@@ -83,7 +83,8 @@ def test_few_rows(M, N, K):
     assert _lib.read_status() == 0
 
 
-@pytest.mark.parametrize("M,N,K", [(5000, 4104, 64), (9001, 776, 136), (20000, 264, 200), (2500, 6000, 256), (19000, 520, 328)])
+@pytest.mark.parametrize("M,N,K", [(5000, 4104, 64), (9001, 776, 136), (20000, 264, 200), (2500, 6000, 256), (19000, 520, 328),
+                                   (300, 136, 72), (600, 2056, 520), (9472, 264, 264), (4000, 1544, 4104)])
 def test_wide_tiles(M, N, K):
     """The 256 x 512 pair tiles at their edges: one to six blocks of the reduction (the second column block starts up to three
     late), ragged rows and columns, a last wave cut into column halves, every operand layout, stores and accumulation in
