@@ -578,7 +578,7 @@ int halo_gemm_bf16(const void* A, const void* B, void* C, void* aux, int M, int 
     //    reductions from 512 to 2048 (8192 x 2 x 6144, K = 256 / 512 / 2048 / 4096  86 / 117 / 325 / 595 against 94 / 104 / 295 / 639).
     //  * bf16 +=: the lanes read and write C themselves, and the wide kernel has no second tile to do it under
     //    (16384 x 12288 x 4096  1,746 / 1,312; 4096 x 24576 x 8192  1,168 / 1,354).
-    // Over 4,860 shapes timed on both sides (all stores but fp32 +=, which the wide kernel is never slower at) the chosen kernel is
+    // Over 4,860 shapes timed on both sides (all stores but fp32 +=, which the wide kernel is hardly ever slower at) the chosen kernel is
     // within 0.7 % of the better one on average; by the waves alone 3.3 %.
     const long long single_tiles = (long long)p.tiles_m * p.tiles_n;
     const bool stores = epi == kEpiStoreBf16 || epi == kEpiStoreF32;
