@@ -181,13 +181,33 @@ adamw_bf16_kernel(AdamTable tab, AdamSingle one, float beta1, float beta2, float
         }
         return;
     }
-    // the last block of a tensor, and tensors that do not start on 16-byte boundaries
+    // The last block of a tensor, and tensors that do not start on 16-byte boundaries: four elements a thread and step, in 8-byte
+    // pieces where the boundaries allow (60 M parameters on 8-byte boundaries: 333 us element by element).
+    const bool halves = (((uintptr_t)p | (uintptr_t)m | (uintptr_t)v | (GRAD_F32 ? 0 : (uintptr_t)gptr)) & 7u) == 0;
 #pragma unroll 1
     for (int it = 0; it < 2 * kIters; ++it) {
         const long long quad = (chunk0 >> 2) + (long long)it * kAdamThreads + threadIdx.x;
         const long long e0 = quad * 4;
         if (e0 >= n) break;
         const Philox rnd = philox4x32_10(k0, k1, (uint32_t)quad, (uint32_t)((unsigned long long)quad >> 32));
+        if (halves && e0 + 4 <= n) {
+            uint2 pc = *reinterpret_cast<const uint2*>(p + e0), mc = *reinterpret_cast<const uint2*>(m + e0);
+            uint2 vc = *reinterpret_cast<const uint2*>(v + e0), gc = make_uint2(0, 0);
+            if (!GRAD_F32) gc = *reinterpret_cast<const uint2*>((const __nv_bfloat16*)gptr + e0);
+            __nv_bfloat16* ph = reinterpret_cast<__nv_bfloat16*>(&pc);
+            __nv_bfloat16* mh = reinterpret_cast<__nv_bfloat16*>(&mc);
+            __nv_bfloat16* vh = reinterpret_cast<__nv_bfloat16*>(&vc);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float g = GRAD_F32 ? ((const float*)gptr)[e0 + j] : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(&gc)[j]);
+                adam_element<GRAD_F32>(k, has_scale, rnd.c[j], __bfloat162float(ph[j]), __bfloat162float(mh[j]), __bfloat162float(vh[j]), g,
+                                       ph[j], mh[j], vh[j]);
+            }
+            *reinterpret_cast<uint2*>(p + e0) = pc;
+            *reinterpret_cast<uint2*>(m + e0) = mc;
+            *reinterpret_cast<uint2*>(v + e0) = vc;
+            continue;
+        }
         for (int j = 0; j < 4 && e0 + j < n; ++j) {
             const float g = GRAD_F32 ? ((const float*)gptr)[e0 + j] : __bfloat162float(((const __nv_bfloat16*)gptr)[e0 + j]);
             __nv_bfloat16 po, mo, vo;

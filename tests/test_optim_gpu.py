@@ -151,7 +151,7 @@ def test_adamw_q8_kernel_equals_its_tensor_op_statement(grad_dtype):
     assert all(torch.equal(a, pg) for a, (_, pg) in zip(before, gpu))
 
 
-@pytest.mark.parametrize("numel,offset", [(7, 0), (16384, 0), (16385, 8), (40000, 1), (50003, 4)])
+@pytest.mark.parametrize("numel,offset", [(7, 0), (16384, 0), (16385, 8), (40000, 1), (50003, 4), (20002, 12), (9, 4)])
 def test_adamw_blocks_and_alignment(numel, offset):
     """Whole blocks, the ragged last one and tensors off the 16-byte boundary, with zero and overflowing gradients, bit
     for bit against the CPU statement."""
