@@ -100,10 +100,24 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 }
 
 // The same for a whole converged warp, with one answer for all its lanes: a lane that gave up alone would leave the others in
-// the next warp-wide instruction or barrier, which has no limit.
+// the next warp-wide instruction or barrier, which has no limit. The lanes poll together, so that the common case is one try,
+// one vote and no divergent branch (a vote behind the per-lane wait cost the attention forward 1.3 %).
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status,
                                                uint64_t budget_ns = HALO_WAIT_BUDGET_NS) {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, budget_ns));
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    const uint64_t t0 = global_timer_ns();
+    uint32_t spins = 0;
+    while (true) {
+        if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+        if ((++spins & 255u) == 0u) {
+            const bool late = global_timer_ns() - t0 > budget_ns;
+            if (late) {
+                *abort_flag = 1;
+                if (status) atomicCAS(status, kStatusOk, kStatusWaitTimeout);
+            }
+            if (__any_sync(0xffffffffu, late || *abort_flag != 0)) return false;
+        }
+    }
 }
 // Whether a whole converged warp should stop: one answer for all its lanes.
 __device__ __forceinline__ bool warp_aborted(const volatile int* abort_flag) {
