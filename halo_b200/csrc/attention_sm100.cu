@@ -29,7 +29,6 @@ constexpr float kLog2e = 1.4426950408889634f;
 int make_tmap_bf16(CUtensorMap* m, const void* base, long long rows, long long cols, long long ld,
                    int box_rows);  // gemm_sm100.cu
 
-// 2^x on the special-function unit (one MUFU op; inputs here are <= 8 after max subtraction)
 // (x.x * m + a, x.y * m + a) in one packed operation
 __device__ __forceinline__ float2 fma2(float2 x, float m, float a) {
     float2 r;
@@ -39,6 +38,7 @@ __device__ __forceinline__ float2 fma2(float2 x, float m, float a) {
         : "=f"(r.x), "=f"(r.y) : "f"(x.x), "f"(x.y), "f"(m), "f"(a));
     return r;
 }
+// 2^x on the special-function unit (one MUFU op; inputs here are <= 8 after max subtraction)
 __device__ __forceinline__ float fast_exp2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
