@@ -198,37 +198,41 @@ def test_accumulate_keeps_subnormals_and_neighbours(m, n):
     assert torch.equal(buf.view(torch.int32), before.view(torch.int32))
 
 
-def test_few_rows_from_two_threads():
-    """Two threads on streams of their own, one with the smallest tile's ring and one with the largest: a launch gets the
-    shared memory it asks for whatever the other thread's call sets in between."""
+def test_few_rows_from_several_threads():
+    """Threads on streams of their own, some with the smallest tile's ring and some with the largest: a launch gets the
+    shared memory it asks for whatever another thread's call sets in between. The entry point is called bare, so that the
+    threads meet inside it and not at the interpreter's lock."""
     import threading
 
     from halo_b200.ops import _lib
-    from halo_b200.ops.gemm import matmul
 
     torch.manual_seed(0)
-    w = torch.randn(512, 4096, device="cuda").bfloat16()
+    N, K = 512, 4096
+    w = torch.randn(N, K, device="cuda").bfloat16()
+    entry = _lib.lib()._cdll.halo_gemm_bf16
+    jobs = []
+    for rows in (16, 200, 16, 200):
+        x, out = torch.ones(rows, K, device="cuda").bfloat16(), torch.empty(rows, N, device="cuda", dtype=torch.bfloat16)
+        stream = torch.cuda.Stream()
+        args = (_lib.ptr(x), _lib.ptr(w), _lib.ptr(out), _lib.c_void_p(0), _lib.c_int(rows), _lib.c_int(N), _lib.c_int(K), _lib.c_ll(K),
+                _lib.c_ll(K), _lib.c_ll(N), _lib.c_ll(0), _lib.c_int(0), _lib.c_int(0), _lib.c_int(0), _lib.c_float(1.0),
+                _lib.ptr(_lib.status_word(w.device)), _lib.c_void_p(stream.cuda_stream))
+        jobs.append((x, out, stream, args))
     torch.cuda.synchronize()
-    failures = []
+    codes = []
 
-    def work(rows):
-        try:
-            x = torch.ones(rows, 4096, device="cuda").bfloat16()
-            with torch.cuda.stream(torch.cuda.Stream()):
-                torch.cuda.current_stream().wait_stream(torch.cuda.default_stream())
-                out = torch.empty(rows, 512, device="cuda", dtype=torch.bfloat16)
-                for _ in range(4000):
-                    matmul(x, w, out=out)
-                torch.cuda.current_stream().synchronize()
-            want = w.double().sum(1)
-            assert ((out - want).abs() <= 2.0 ** -8 * want.abs() + 0.05).all()
-        except BaseException as exc:
-            failures.append(exc)
+    def work(args):
+        torch.cuda.set_device(0)
+        codes.extend({entry(*args) for _ in range(5000)})
 
-    threads = [threading.Thread(target=work, args=(rows,)) for rows in (16, 200)]
+    threads = [threading.Thread(target=work, args=(job[3],)) for job in jobs]
     for t in threads:
         t.start()
     for t in threads:
         t.join()
-    assert not failures, failures
+    torch.cuda.synchronize()
+    assert codes == [0] * len(jobs), codes
+    want = w.double().sum(1)
+    for _, out, _, _ in jobs:
+        assert ((out - want).abs() <= 2.0 ** -8 * want.abs() + 0.05).all()
     assert _lib.read_status() == 0
