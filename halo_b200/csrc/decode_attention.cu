@@ -31,13 +31,24 @@ namespace halo {
 namespace decode {
 
 constexpr int kWarps = 4;
+constexpr unsigned kMaxGridZ = 65535;
 constexpr int kMaxGroup = 16;      // query heads per key/value head
 constexpr int kTileKeys = 16;      // keys per warp and step
 constexpr int kStages = 3;         // ring depth per warp: 2 blocks of 96 KB per SM keep 128 KB of loads in flight
 
+// 16 bytes of the cache; in four pieces where its rows do not start on 16-byte boundaries (A16 false)
+template <bool A16>
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool live) {
-    const int bytes = live ? 16 : 0;    // 0: the 16 bytes are filled with zeros, nothing is read
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+    if (A16) {
+        const int bytes = live ? 16 : 0;    // 0: the 16 bytes are filled with zeros, nothing is read
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+    } else {
+        const int bytes = live ? 4 : 0;
+#pragma unroll
+        for (int i = 0; i < 16; i += 4)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + i),
+                         "l"(reinterpret_cast<const uint8_t*>(src) + i), "r"(bytes) : "memory");
+    }
 }
 __device__ __forceinline__ void ldmatrix4(uint32_t a, uint32_t (&r)[4]) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
@@ -68,19 +79,21 @@ template <int D>
 __host__ __device__ constexpr int state_floats() { return 2 * kMaxGroup + kMaxGroup * D; }
 
 // SPLIT2: groups of more than 8 heads use all 16 rows of the product, so the low terms need a product of their own
-template <int D, bool SPLIT2>
+template <int D, bool SPLIT2, bool A16>
 __global__ void __launch_bounds__(kWarps * 32, 2)
 decode_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ kc,
                         const __nv_bfloat16* __restrict__ vc, const long long* __restrict__ cols,
                         __nv_bfloat16* __restrict__ out, int n_heads, int n_kv_heads, long long max_len, float scale,
-                        int parts) {
+                        int parts, int batch) {
     static_assert(kWarps * state_floats<D>() * 4 <= ring_bytes<D>(), "the partial states fit over the ring");
     extern __shared__ __align__(128) uint8_t smem[];
     const uint32_t base = smem_u32(smem);
     constexpr int kRow = D * 2;                     // bytes of a key
     constexpr int kTile = kTileKeys * kRow;         // bytes of a warp's key (or value) tile
     constexpr int kChunks = D / 8;                  // 16-byte chunks per row
-    const int b = blockIdx.z, hk = blockIdx.y;
+    const int hk = blockIdx.y;
+    const long long b = blockIdx.z + (long long)(blockIdx.x / parts) * gridDim.z;       // x holds several only above 65,535 sequences
+    if (b >= batch) return;                         // the whole cluster
     const uint32_t part = cluster_cta_rank();
     const int G = n_heads / n_kv_heads;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -95,8 +108,8 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
     const int mine = (int)max(0ll, (tile_hi - tile_lo - warp + kWarps - 1) / kWarps);   // tiles tile_lo + warp + 4 i
 
     const long long key_stride = (long long)n_kv_heads * D;
-    const __nv_bfloat16* kb = kc + (long long)b * max_len * key_stride + (long long)hk * D;
-    const __nv_bfloat16* vb = vc + (long long)b * max_len * key_stride + (long long)hk * D;
+    const __nv_bfloat16* kb = kc + b * max_len * key_stride + (long long)hk * D;
+    const __nv_bfloat16* vb = vc + b * max_len * key_stride + (long long)hk * D;
     const uint32_t ring = base + warp * (kStages * 2 * kTile);
 
     auto load_tile = [&](int i) {
@@ -109,8 +122,8 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
                 const bool live = k0 + r < n_keys;
                 const long long off = (live ? k0 + r : 0) * key_stride + ch * 8;
                 const uint32_t d = dst + r * kRow + ((ch ^ (r & 7)) << 4);     // chunks swizzled by row
-                cp_async16(d, kb + off, live);
-                cp_async16(d + kTile, vb + off, live);
+                cp_async16<A16>(d, kb + off, live);
+                cp_async16<A16>(d + kTile, vb + off, live);
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");                   // empty groups keep the count uniform
@@ -121,7 +134,7 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
     // query fragments: row g is head g (and g + 8: the head again, so that its low terms find their scores in place)
     uint32_t qa[D / 16][4];
     {
-        const __nv_bfloat16* qb = q + ((long long)b * n_heads + (long long)hk * G) * D;
+        const __nv_bfloat16* qb = q + (b * n_heads + (long long)hk * G) * D;
         const int r0 = g, r1 = SPLIT2 ? g + 8 : g;
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks) {
@@ -315,19 +328,20 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
             nb += ld_cluster(base + 4 * (2 * kMaxGroup + e + 1), c) * f;
         }
         const float inv = 1.f / den;
-        *reinterpret_cast<uint32_t*>(out + ((long long)b * n_heads + (long long)hk * G) * D + e) = pack_bf16(na * inv, nb * inv);
+        *reinterpret_cast<uint32_t*>(out + (b * n_heads + (long long)hk * G) * D + e) = pack_bf16(na * inv, nb * inv);
     }
     cluster_sync_all();                                 // nobody leaves while its state is still being read
 }
 
-template <int D, bool SPLIT2>
+template <int D, bool SPLIT2, bool A16>
 static int launch(const void* q, const void* kc, const void* vc, const long long* cols, void* out, int batch, int n_heads,
                   int n_kv_heads, long long max_len, float scale, int parts, cudaStream_t s) {
-    auto kernel = decode_attention_kernel<D, SPLIT2>;
+    auto kernel = decode_attention_kernel<D, SPLIT2, A16>;
     // set for the current device at every launch: the call costs well under a microsecond and keeps no state here
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ring_bytes<D>()) != cudaSuccess) return -10;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)parts, (unsigned)n_kv_heads, (unsigned)batch);
+    const unsigned z = batch < kMaxGridZ ? batch : kMaxGridZ;
+    cfg.gridDim = dim3(parts * ((batch + z - 1) / z), (unsigned)n_kv_heads, z);
     cfg.blockDim = dim3(kWarps * 32, 1, 1);
     cfg.dynamicSmemBytes = ring_bytes<D>();
     cfg.stream = s;
@@ -340,12 +354,17 @@ static int launch(const void* q, const void* kc, const void* vc, const long long
     cfg.numAttrs = 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, (const __nv_bfloat16*)q, (const __nv_bfloat16*)kc,
                                              (const __nv_bfloat16*)vc, cols, (__nv_bfloat16*)out, n_heads, n_kv_heads, max_len,
-                                             scale, parts);
+                                             scale, parts, batch);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return -11;
     }
     return 0;
+}
+
+template <int D, bool SPLIT2, typename... Args>
+static int launch_form(bool a16, Args... args) {
+    return a16 ? launch<D, SPLIT2, true>(args...) : launch<D, SPLIT2, false>(args...);
 }
 
 }  // namespace decode
@@ -354,15 +373,15 @@ static int launch(const void* q, const void* kc, const void* vc, const long long
 extern "C" {
 
 // q, out: [batch, n_heads * head_dim] bf16 contiguous. kc, vc: one layer of the cache, [batch, max_len, n_kv_heads,
-// head_dim] bf16 contiguous. cols: [batch] int64 on the device.
+// head_dim] bf16 contiguous, on 4-byte boundaries. cols: [batch] int64 on the device.
 int halo_decode_attention(const void* q, const void* kc, const void* vc, const long long* cols, void* out, int batch,
                           int n_heads, int n_kv_heads, int head_dim, long long max_len, float scale, void* stream) {
     using namespace halo::decode;
     if (batch < 0 || n_kv_heads < 1 || n_heads % n_kv_heads || n_heads / n_kv_heads > kMaxGroup || max_len < 1) return -1;
     if (head_dim != 128 && head_dim != 64) return -1;
     if (batch == 0) return 0;
-    if (batch > 65535 || n_kv_heads > 65535) return -1;
-    if ((reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 15u) return -2;   // 16-byte copies
+    if (n_kv_heads > 65535) return -1;
+    if ((reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 3u) return -2;
     cudaStream_t s = (cudaStream_t)stream;
     // Parts per (sequence, key/value head). The SMs hold 296 blocks, and a part below 128 keys is all merge; up to 4 parts while
     // the grid stays below two waves (measured at 64 sequences of 8,000 keys: 1 / 2 / 4 / 8 parts 119 / 115 / 106 / 122 us; at
@@ -373,11 +392,12 @@ int halo_decode_attention(const void* q, const void* kc, const void* vc, const l
     int parts = 1;
     while (parts < most && pairs * parts < 592 && max_len > 128ll * parts) parts *= 2;
     const bool split2 = n_heads / n_kv_heads > 8;
+    const bool a16 = ((reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 15u) == 0;
     if (head_dim == 128)
-        return split2 ? launch<128, true>(q, kc, vc, cols, out, batch, n_heads, n_kv_heads, max_len, scale, parts, s)
-                      : launch<128, false>(q, kc, vc, cols, out, batch, n_heads, n_kv_heads, max_len, scale, parts, s);
-    return split2 ? launch<64, true>(q, kc, vc, cols, out, batch, n_heads, n_kv_heads, max_len, scale, parts, s)
-                  : launch<64, false>(q, kc, vc, cols, out, batch, n_heads, n_kv_heads, max_len, scale, parts, s);
+        return split2 ? launch_form<128, true>(a16, q, kc, vc, cols, out, batch, n_heads, n_kv_heads, max_len, scale, parts, s)
+                      : launch_form<128, false>(a16, q, kc, vc, cols, out, batch, n_heads, n_kv_heads, max_len, scale, parts, s);
+    return split2 ? launch_form<64, true>(a16, q, kc, vc, cols, out, batch, n_heads, n_kv_heads, max_len, scale, parts, s)
+                  : launch_form<64, false>(a16, q, kc, vc, cols, out, batch, n_heads, n_kv_heads, max_len, scale, parts, s);
 }
 
 }  // extern "C"

@@ -390,3 +390,34 @@ def test_cached_attention_takes_the_positions_an_index_expression_takes(form):
     keys[rows, cols] = k.view(T, kv_heads, 128)
     values[rows, cols] = v.reshape(T, kv_heads, 128)
     assert torch.equal(got, want) and torch.equal(cache.k[0], keys) and torch.equal(cache.v[0], values) and _lib.read_status() == 0
+
+
+def _decode_reference(cache, q, heads):
+    from halo_b200.inference.generate import KVCache
+
+    _, B, S, kv_heads, D = cache.k.shape
+    ref = KVCache(1, B, S, kv_heads, D, torch.float64, "cuda")
+    ref.k.copy_(cache.k)
+    ref.v.copy_(cache.v)
+    ref.lengths.copy_(cache.lengths)
+    ref.begin_decode()
+    return ref.attend(0, q.double(), heads)
+
+
+@pytest.mark.parametrize("B,S,heads,kv_heads,D,shift", [(5, 300, 8, 2, 128, 4), (3, 70, 12, 2, 64, 2), (70, 530, 8, 1, 64, 6), (66000, 3, 2, 1, 64, 0),
+                                                       (65536, 2, 1, 1, 64, 2)])
+def test_decode_attention_takes_any_cache_and_batch(B, S, heads, kv_heads, D, shift):
+    """Caches that start on 4- or 8-byte boundaries and more sequences than one grid dimension has room for. One bf16
+    rounding of the output and fp32 noise, as for every decode call."""
+    from halo_b200.inference.generate import KVCache
+    from halo_b200.ops import _lib
+
+    torch.manual_seed(S)
+    cache = KVCache(1, B, S, kv_heads, D, torch.bfloat16, "cuda")
+    n = cache.k.numel()
+    cache.k, cache.v = (torch.randn(n + shift, device="cuda").bfloat16()[shift:].view(cache.k.shape) for _ in range(2))
+    cache.lengths.copy_(torch.randint(0, S, (B,)))
+    cache.begin_decode()
+    q = torch.randn(B, heads * D, device="cuda").bfloat16()
+    got, want = cache.attend(0, q, heads).double(), _decode_reference(cache, q, heads)
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all() and _lib.read_status() == 0
