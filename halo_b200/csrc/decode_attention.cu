@@ -18,7 +18,8 @@
 // free: the product has 16 rows, the heads use rows 0-7 and the low terms ride in rows 8-15.
 //
 // Measured (B200, 64 sequences of 2,000-8,000 keys, 32 / 4 heads of 128: 655 MB of cache): 3,662 us before (one block of
-// four warps per pair, shuffles and scalar products), 106 us now = 6.1 TB/s of cache (0.93 of the measured copy rate).
+// four warps per pair, shuffles and scalar products), 109 us now = 6.0 TB/s of cache (0.92 of the measured copy rate).
+// Against 64 bits the error of the bf16 output is the former kernel's in seven digits (14 shapes, flat and sharp softmax).
 //
 // Sequence lengths are read on the device - the host never synchronises on them.
 // Stands where the reference's rollout engines run their paged decode kernels; here the cache is the sampler's own
@@ -30,7 +31,6 @@
 namespace halo {
 namespace decode {
 
-constexpr int kWarps = 4;
 constexpr unsigned kMaxGridZ = 65535;
 constexpr int kMaxGroup = 16;      // query heads per key/value head
 constexpr int kTileKeys = 16;      // keys per warp and step
@@ -72,20 +72,21 @@ __device__ __forceinline__ float ld_cluster(uint32_t local_addr, uint32_t rank) 
     return v;
 }
 
-template <int D>
-__host__ __device__ constexpr int ring_bytes() { return kWarps * kStages * kTileKeys * D * 2 * 2; }
+template <int D, int WARPS>
+__host__ __device__ constexpr int ring_bytes() { return WARPS * kStages * kTileKeys * D * 2 * 2; }
 // per-warp partial states, laid over the ring once the loop is over: m, l [kMaxGroup] and acc [kMaxGroup][D] fp32
 template <int D>
 __host__ __device__ constexpr int state_floats() { return 2 * kMaxGroup + kMaxGroup * D; }
 
-// SPLIT2: groups of more than 8 heads use all 16 rows of the product, so the low terms need a product of their own
-template <int D, bool SPLIT2, bool A16>
-__global__ void __launch_bounds__(kWarps * 32, 2)
+// SPLIT2: groups of more than 8 heads use all 16 rows of the product, so the low terms need a product of their own.
+// WARPS: 4, or 1 for caches of few keys (see the entry point).
+template <int D, bool SPLIT2, int WARPS, bool A16>
+__global__ void __launch_bounds__(WARPS * 32, 8 / WARPS)
 decode_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ kc,
                         const __nv_bfloat16* __restrict__ vc, const long long* __restrict__ cols,
                         __nv_bfloat16* __restrict__ out, int n_heads, int n_kv_heads, long long max_len, float scale,
                         int parts, int batch) {
-    static_assert(kWarps * state_floats<D>() * 4 <= ring_bytes<D>(), "the partial states fit over the ring");
+    static_assert(WARPS * state_floats<D>() * 4 <= ring_bytes<D, WARPS>(), "the partial states fit over the ring");
     extern __shared__ __align__(128) uint8_t smem[];
     const uint32_t base = smem_u32(smem);
     constexpr int kRow = D * 2;                     // bytes of a key
@@ -105,7 +106,7 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
     const long long tiles = (n_keys + kTileKeys - 1) / kTileKeys;
     const long long share = (tiles + parts - 1) / parts;
     const long long tile_lo = min(tiles, share * part), tile_hi = min(tiles, tile_lo + share);
-    const int mine = (int)max(0ll, (tile_hi - tile_lo - warp + kWarps - 1) / kWarps);   // tiles tile_lo + warp + 4 i
+    const int mine = (int)max(0ll, (tile_hi - tile_lo - warp + WARPS - 1) / WARPS);   // tiles tile_lo + warp + 4 i
 
     const long long key_stride = (long long)n_kv_heads * D;
     const __nv_bfloat16* kb = kc + b * max_len * key_stride + (long long)hk * D;
@@ -114,7 +115,7 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
 
     auto load_tile = [&](int i) {
         if (i < mine) {
-            const long long k0 = (tile_lo + warp + (long long)i * kWarps) * kTileKeys;
+            const long long k0 = (tile_lo + warp + (long long)i * WARPS) * kTileKeys;
             const uint32_t dst = ring + (i % kStages) * 2 * kTile;
 #pragma unroll
             for (int c = 0; c < kTileKeys * kChunks / 32; ++c) {
@@ -158,7 +159,7 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
         asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 1) : "memory");
         __syncwarp();
         const uint32_t sk = ring + (i % kStages) * 2 * kTile, sv = sk + kTile;
-        const long long k0 = (tile_lo + warp + (long long)i * kWarps) * kTileKeys;
+        const long long k0 = (tile_lo + warp + (long long)i * WARPS) * kTileKeys;
         float s[2][4];                              // scores: keys 0-7 and 8-15 of the tile
 #pragma unroll
         for (int n = 0; n < 2; ++n)
@@ -284,15 +285,36 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
         }
     }
     __syncthreads();
+    __nv_bfloat16* out_rows = out + (b * n_heads + (long long)hk * G) * D;
+    if (parts == 1) {                                   // the block's warps are all there is to merge
+        for (int e = 2 * threadIdx.x; e < G * D; e += 2 * WARPS * 32) {
+            const int h = e / D;
+            float big = -INFINITY;
+#pragma unroll
+            for (int w = 0; w < WARPS; ++w) big = fmaxf(big, st[w * state_floats<D>() + h]);
+            float den = 0.f, na = 0.f, nb = 0.f;
+#pragma unroll
+            for (int w = 0; w < WARPS; ++w) {
+                const float* sw = st + w * state_floats<D>();
+                const float f = sw[h] == -INFINITY ? 0.f : exp2f(sw[h] - big);     // a warp that saw no key: weight 0
+                den += sw[kMaxGroup + h] * f;
+                na += sw[2 * kMaxGroup + e] * f;
+                nb += sw[2 * kMaxGroup + e + 1] * f;
+            }
+            const float inv = 1.f / den;
+            *reinterpret_cast<uint32_t*>(out_rows + e) = pack_bf16(na * inv, nb * inv);
+        }
+        return;
+    }
     // fold the block's warps into warp 0's slot: element (head, d) belongs to one thread, the statistics are read first
-    for (int e = threadIdx.x; e < G * D; e += kWarps * 32) {
+    for (int e = threadIdx.x; e < G * D; e += WARPS * 32) {
         const int h = e / D;
         float big = -INFINITY;
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) big = fmaxf(big, st[w * state_floats<D>() + h]);
+        for (int w = 0; w < WARPS; ++w) big = fmaxf(big, st[w * state_floats<D>() + h]);
         float num = 0.f;
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
+        for (int w = 0; w < WARPS; ++w) {
             const float mw = st[w * state_floats<D>() + h];
             const float f = mw == -INFINITY ? 0.f : exp2f(mw - big);   // a warp that saw no key: weight 0
             num += st[w * state_floats<D>() + 2 * kMaxGroup + e] * f;
@@ -304,9 +326,9 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
         const int h = threadIdx.x;
         float big = -INFINITY, den = 0.f;
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) big = fmaxf(big, st[w * state_floats<D>() + h]);
+        for (int w = 0; w < WARPS; ++w) big = fmaxf(big, st[w * state_floats<D>() + h]);
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
+        for (int w = 0; w < WARPS; ++w) {
             const float mw = st[w * state_floats<D>() + h];
             den += mw == -INFINITY ? 0.f : st[w * state_floats<D>() + kMaxGroup + h] * exp2f(mw - big);
         }
@@ -315,7 +337,7 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
     }
     __syncthreads();
     cluster_sync_all();                                 // every part's state is in its block's shared memory
-    for (int e = 2 * (part * (kWarps * 32) + threadIdx.x); e < G * D; e += 2 * parts * (kWarps * 32)) {
+    for (int e = 2 * (part * (WARPS * 32) + threadIdx.x); e < G * D; e += 2 * parts * (WARPS * 32)) {
         const int h = e / D;
         float big = -INFINITY;
         for (int c = 0; c < parts; ++c) big = fmaxf(big, ld_cluster(base + 4 * h, c));
@@ -328,22 +350,32 @@ decode_attention_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
             nb += ld_cluster(base + 4 * (2 * kMaxGroup + e + 1), c) * f;
         }
         const float inv = 1.f / den;
-        *reinterpret_cast<uint32_t*>(out + (b * n_heads + (long long)hk * G) * D + e) = pack_bf16(na * inv, nb * inv);
+        *reinterpret_cast<uint32_t*>(out_rows + e) = pack_bf16(na * inv, nb * inv);
     }
     cluster_sync_all();                                 // nobody leaves while its state is still being read
 }
 
-template <int D, bool SPLIT2, bool A16>
+static int num_sms() {                  // asked once: every GPU of a machine has as many
+    static const int n = [] {
+        int dev = 0, v = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) v = 0;
+        return v > 0 ? v : 148;
+    }();
+    return n;
+}
+
+template <int D, bool SPLIT2, int WARPS, bool A16>
 static int launch(const void* q, const void* kc, const void* vc, const long long* cols, void* out, int batch, int n_heads,
                   int n_kv_heads, long long max_len, float scale, int parts, cudaStream_t s) {
-    auto kernel = decode_attention_kernel<D, SPLIT2, A16>;
+    auto kernel = decode_attention_kernel<D, SPLIT2, WARPS, A16>;
+    constexpr int kSmem = ring_bytes<D, WARPS>();
     // set for the current device at every launch: the call costs well under a microsecond and keeps no state here
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ring_bytes<D>()) != cudaSuccess) return -10;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess) return -10;
     cudaLaunchConfig_t cfg = {};
     const unsigned z = batch < kMaxGridZ ? batch : kMaxGridZ;
     cfg.gridDim = dim3(parts * ((batch + z - 1) / z), (unsigned)n_kv_heads, z);
-    cfg.blockDim = dim3(kWarps * 32, 1, 1);
-    cfg.dynamicSmemBytes = ring_bytes<D>();
+    cfg.blockDim = dim3(WARPS * 32, 1, 1);
+    cfg.dynamicSmemBytes = kSmem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -363,8 +395,9 @@ static int launch(const void* q, const void* kc, const void* vc, const long long
 }
 
 template <int D, bool SPLIT2, typename... Args>
-static int launch_form(bool a16, Args... args) {
-    return a16 ? launch<D, SPLIT2, true>(args...) : launch<D, SPLIT2, false>(args...);
+static int launch_form(int warps, bool a16, Args... args) {
+    if (!a16) return launch<D, SPLIT2, 4, false>(args...);
+    return warps == 1 ? launch<D, SPLIT2, 1, true>(args...) : launch<D, SPLIT2, 4, true>(args...);
 }
 
 }  // namespace decode
@@ -383,21 +416,29 @@ int halo_decode_attention(const void* q, const void* kc, const void* vc, const l
     if (n_kv_heads > 65535) return -1;
     if ((reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 3u) return -2;
     cudaStream_t s = (cudaStream_t)stream;
-    // Parts per (sequence, key/value head). The SMs hold 296 blocks, and a part below 128 keys is all merge; up to 4 parts while
-    // the grid stays below two waves (measured at 64 sequences of 8,000 keys: 1 / 2 / 4 / 8 parts 119 / 115 / 106 / 122 us; at
-    // 16 x 4,000: 42 / - / 21 / 27 us). Wider clusters wait for eight free blocks in one GPC at a time and lose, except where
-    // even then no SM gets a second block (2 sequences of 8,000 keys: 4 parts 17.7 us, 8 parts 12.8 us; 16 parts 13.7 us).
-    const long long pairs = (long long)batch * n_kv_heads;
-    const int most = pairs * 8 <= 148 ? 8 : 4;
+    // Parts per (sequence, key/value head) and warps per block. `wave` blocks of four warps run at once, and every further part
+    // costs a cluster, its barriers and a merge, whatever the sequences hold (64 sequences of 4 such heads, 1 / 2 / 4 parts, us:
+    // 30 keys each 6 / 14 / 25; caches of 1,024, ragged, 20 / 28 / 37; of 4,000 62 / 66 / 66; of 8,000 117 / 120 / 110).
+    //  * Caches below 400 keys are not cut.
+    //  * Longer ones are cut to fill one wave, and from 3,000 keys on beyond it, for then the longest of a ragged batch decides.
+    //  * Eight parts wait for eight free blocks in one GPC at a time and lose, except where even then no SM gets a second block
+    //    (2 sequences of 8,000 keys: 4 / 8 parts 23 / 16 us).
+    //  * More pairs than one and a half waves over caches of at most 500 keys: one-warp blocks, of which nine fit an SM and which
+    //    have no merge at all (1,000 sequences of 4 heads, 4 / 1 warps: 1 key each 47 / 20, 300 keys 110 / 104).
+    const int sms = num_sms();
+    const long long pairs = (long long)batch * n_kv_heads, wave = 2ll * sms;
+    const int most = pairs * 8 <= sms ? 8 : 4;
     int parts = 1;
-    while (parts < most && pairs * parts < 592 && max_len > 128ll * parts) parts *= 2;
+    if (max_len >= 400)
+        while (parts < most && pairs * parts < 2 * wave && max_len > 128ll * parts && (pairs * parts * 2 <= wave || max_len >= 3000)) parts *= 2;
+    const int warps = parts == 1 && 2 * pairs > 3 * wave && max_len <= 500 ? 1 : 4;
     const bool split2 = n_heads / n_kv_heads > 8;
     const bool a16 = ((reinterpret_cast<uintptr_t>(kc) | reinterpret_cast<uintptr_t>(vc)) & 15u) == 0;
     if (head_dim == 128)
-        return split2 ? launch_form<128, true>(a16, q, kc, vc, cols, out, batch, n_heads, n_kv_heads, max_len, scale, parts, s)
-                      : launch_form<128, false>(a16, q, kc, vc, cols, out, batch, n_heads, n_kv_heads, max_len, scale, parts, s);
-    return split2 ? launch_form<64, true>(a16, q, kc, vc, cols, out, batch, n_heads, n_kv_heads, max_len, scale, parts, s)
-                  : launch_form<64, false>(a16, q, kc, vc, cols, out, batch, n_heads, n_kv_heads, max_len, scale, parts, s);
+        return split2 ? launch_form<128, true>(warps, a16, q, kc, vc, cols, out, batch, n_heads, n_kv_heads, max_len, scale, parts, s)
+                      : launch_form<128, false>(warps, a16, q, kc, vc, cols, out, batch, n_heads, n_kv_heads, max_len, scale, parts, s);
+    return split2 ? launch_form<64, true>(warps, a16, q, kc, vc, cols, out, batch, n_heads, n_kv_heads, max_len, scale, parts, s)
+                  : launch_form<64, false>(warps, a16, q, kc, vc, cols, out, batch, n_heads, n_kv_heads, max_len, scale, parts, s);
 }
 
 }  // extern "C"

@@ -145,7 +145,8 @@ def test_decode_attention_kernel(heads, kv_heads, D):
 
 
 @pytest.mark.parametrize("B,S,heads,kv_heads,D", [(1, 129, 32, 4, 128), (2, 1100, 32, 4, 128), (37, 530, 24, 2, 128), (40, 1030, 12, 4, 64),
-                                                  (150, 700, 8, 4, 128)])
+                                                  (150, 700, 8, 4, 128), (30, 530, 12, 4, 64), (80, 3100, 4, 2, 64), (120, 500, 32, 4, 128),
+                                                  (450, 20, 24, 2, 128), (500, 33, 1, 1, 64), (149, 17, 8, 4, 64)])
 def test_decode_attention_parts(B, S, heads, kv_heads, D):
     """Every split of the keys over blocks (1, 2, 4 and 8 parts, some of them empty), groups above and below eight heads; an
     infinite value stays infinite. The output is rounded to bf16 once: 2^-8 of the value, plus fp32 noise."""
@@ -421,3 +422,19 @@ def test_decode_attention_takes_any_cache_and_batch(B, S, heads, kv_heads, D, sh
     q = torch.randn(B, heads * D, device="cuda").bfloat16()
     got, want = cache.attend(0, q, heads).double(), _decode_reference(cache, q, heads)
     assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all() and _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("B,S,kv_heads", [(1, 200, 2), (1, 4000, 1), (500, 90, 1)])
+def test_decode_attention_passes_nan_on(B, S, kv_heads):
+    """Sixteen keys that are all NaN fill one warp's tile: its state has no maximum, but its sums are not empty ones."""
+    from halo_b200.inference.generate import KVCache
+
+    torch.manual_seed(B)
+    cache = KVCache(1, B, S, kv_heads, 128, torch.bfloat16, "cuda")
+    cache.k.normal_()
+    cache.v.normal_()
+    cache.k[0, 0, 16:32, 0] = float("nan")
+    cache.lengths.fill_(S - 1)
+    cache.begin_decode()
+    out = cache.attend(0, torch.randn(B, 4 * kv_heads * 128, device="cuda").bfloat16(), 4 * kv_heads).view(B, kv_heads, -1)
+    assert out[0, 0].isnan().all() and out[0, 1:].isfinite().all() and out[1:].isfinite().all()
