@@ -21,7 +21,7 @@ from dataclasses import dataclass, field
 import numpy as np
 import torch
 
-from halo_b200.ops import gemm
+from halo_b200.ops import _lib, gemm
 from halo_b200.ops.norm import rms_norm
 
 
@@ -42,6 +42,14 @@ class Generation:
     logprobs: np.ndarray              # log p(token) under the model's distribution at temperature 1
     finish_reason: str = "length"     # "stop" | "length"
     extra: dict = field(default_factory=dict)
+
+
+def _layer_ptr(cache: torch.Tensor, layer: int):
+    """Where a layer of ``[layers, ...]`` starts, without building the view (which costs as much as a small kernel's launch)."""
+    layers = cache.shape[0]
+    if not -layers <= layer < layers:
+        raise IndexError(f"layer {layer} of a cache of {layers} layers")
+    return _lib.c_void_p(cache.data_ptr() + layer % layers * cache.stride(0) * cache.element_size())
 
 
 class KVCache:
@@ -110,19 +118,17 @@ class KVCache:
         kernel cannot read element by element - on the host, or broadcast over the tokens). Returns ``(q, k or None, layer
         index)``. Negative positions count from the end, as in an index expression; a position outside the cache is skipped
         and recorded in the status word (:func:`halo_b200.ops._lib.raise_on_status`)."""
-        from halo_b200.ops import _lib
-
         cfg = attn.cfg
         Hq, Hkv, D = cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim
         wq, wk = attn.q_norm, attn.k_norm
         T, dev, gpu = qkv.shape[0], qkv.device, qkv.get_device()
-        rows, cols = self._rows, self._cols
-        if (not qkv.is_cuda or D != 128 or qkv.dtype != torch.bfloat16 or T == 0 or qkv.shape[1] != (Hq + 2 * Hkv) * D
-                or self.k.dtype != torch.bfloat16 or self.v.dtype != torch.bfloat16 or self.k.shape[-2:] != (Hkv, D)
-                or self.v.shape != self.k.shape or not self.k.is_contiguous() or not self.v.is_contiguous()
-                or rows.dtype != torch.long or cols.dtype != torch.long or rows.shape != (T,) or cols.shape != (T,)
-                or table.dtype != torch.float32 or table.shape != (T, D // 2, 2)
-                or any(t.get_device() != gpu for t in (self.k, self.v, rows, cols, table))
+        rows, cols, kc, vc = self._rows, self._cols, self.k, self.v
+        if (not qkv.is_cuda or D != 128 or qkv.dtype is not torch.bfloat16 or T == 0 or qkv.shape[1] != (Hq + 2 * Hkv) * D
+                or kc.dtype is not torch.bfloat16 or vc.dtype is not torch.bfloat16 or kc.shape[3] != Hkv or kc.shape[4] != D
+                or vc.shape != kc.shape or not kc.is_contiguous() or not vc.is_contiguous()
+                or rows.dtype is not torch.long or cols.dtype is not torch.long or rows.shape != (T,) or cols.shape != (T,)
+                or table.dtype is not torch.float32 or table.shape != (T, D // 2, 2)
+                or not gpu == kc.get_device() == vc.get_device() == rows.get_device() == cols.get_device() == table.get_device()
                 or (cfg.use_qk_norm and (wq is None or wq.numel() != D)) or not _lib.untransformed()
                 or (torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (qkv, wq, wk)))):
             return None
@@ -133,8 +139,8 @@ class KVCache:
         k = torch.empty((T, Hkv * D), dtype=torch.bfloat16, device=dev) if keep_keys else None
         rows, cols = rows.contiguous(), cols.contiguous()
         rc = _lib.lib().halo_qknorm_rope_cache(
-            _lib.ptr(qkv), _lib.ptr(wq), _lib.ptr(wk), _lib.ptr(table), _lib.ptr(q), _lib.ptr(k), _lib.ptr(self.k[li]),
-            _lib.ptr(self.v[li]), _lib.ptr(rows), _lib.ptr(cols), _lib.c_ll(self.k.shape[1]), _lib.c_ll(self.k.shape[2]),
+            _lib.ptr(qkv), _lib.ptr(wq), _lib.ptr(wk), _lib.ptr(table), _lib.ptr(q), _lib.ptr(k), _layer_ptr(kc, li),
+            _layer_ptr(vc, li), _lib.ptr(rows), _lib.ptr(cols), _lib.c_ll(kc.shape[1]), _lib.c_ll(kc.shape[2]),
             _lib.c_ll(T), _lib.c_int(Hq), _lib.c_int(Hkv), _lib.c_int(D), _lib.c_float(cfg.rms_norm_eps),
             _lib.c_int(1 if cfg.use_qk_norm else 0), _lib.ptr(_lib.status_word(dev)), _lib.stream_ptr(dev))
         _lib.check(rc, "halo_qknorm_rope_cache")
@@ -150,12 +156,10 @@ class KVCache:
         G = n_heads // Hkv
         if q.is_cuda and q.dtype == torch.bfloat16 and D in (64, 128) and G <= 16 and not window and sinks is None and not softcap:
             # the decode kernel streams the cache once and reads the lengths on the device (no host synchronisation)
-            from halo_b200.ops import _lib
-
             qc = q.contiguous()
             out = torch.empty_like(qc)
             rc = _lib.lib().halo_decode_attention(
-                _lib.ptr(qc), _lib.ptr(self.k[li]), _lib.ptr(self.v[li]), _lib.ptr(self._cols), _lib.ptr(out), _lib.c_int(B),
+                _lib.ptr(qc), _layer_ptr(self.k, li), _layer_ptr(self.v, li), _lib.ptr(self._cols), _lib.ptr(out), _lib.c_int(B),
                 _lib.c_int(n_heads), _lib.c_int(Hkv), _lib.c_int(D), _lib.c_ll(self.k.shape[2]),
                 _lib.c_float(scale if scale is not None else D ** -0.5), _lib.stream_ptr(q.device))
             _lib.check(rc, "halo_decode_attention")
