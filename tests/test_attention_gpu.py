@@ -285,3 +285,53 @@ def test_qk_norm_rope_head_counts_and_alignment(T, Hq, Hkv, use_norm, shift):
     want = torch.autograd.grad(y, [xd, wqd, wkd] if use_norm else [xd], torch.cat([gq.view(T, Hq, 128), gk.view(T, Hkv, 128)], 1).double())
     for name, u, v in zip(("dqkv", "dwq", "dwk"), grads, want):
         assert (u - v).norm() <= 2.0 ** -7 * v.norm() + 1e-6, name
+
+
+@pytest.mark.parametrize("direct", [False, True])
+@pytest.mark.parametrize("ranks,lens,balance", [(2, [700, 129, 1, 1218], True), (2, [2048], False), (4, [900, 2300, 896], True)])
+def test_context_parallel_kernels_on_one_gpu(ranks, lens, balance, direct):
+    """The context-parallel instantiations of the attention kernels, every rank's launches one after the other on one GPU
+    with all ranks' buffers in its memory (the kernels themselves never wait for a rank): outputs and gradients against the
+    unsharded attention, with rows mirrored and with tiles read from their owners."""
+    import numpy as np
+
+    from halo_b200.ops import _lib
+    from halo_b200.ops.attention import build_plan, flash_attention
+    from halo_b200.parallel.context_parallel import TILE, CPExchange, build_cp_plan, cp_attention, make_layout
+
+    class OneGpu(CPExchange):
+        def __init__(self, rank, rows, total, cols):
+            self.device, self.n_ranks, self.rank, self.direct_reads = torch.device("cuda", 0), ranks, rank, direct
+            self.kv, self.dkv, self.mirror = (torch.zeros(n, cols, dtype=torch.bfloat16, device="cuda") for n in (rows, total, total))
+            self.mirror_version, self.row_bytes, self.max_local_rows, self.max_row_tokens = 0, cols * 2, rows, total
+
+        def barrier(self):
+            pass
+
+    Hq, Hkv, D = 8, 2, 128
+    cu = np.concatenate([[0], np.cumsum(lens)])
+    T = int(cu[-1])
+    torch.manual_seed(T)
+    q, k, v = _mk(T, Hq, Hkv)
+    do = torch.randn_like(q)
+    leaves = [t.clone().requires_grad_() for t in (q, k, v)]
+    ref = flash_attention(*leaves, build_plan(cu, device="cuda"), Hq, Hkv)
+    want = [ref.detach(), *torch.autograd.grad(ref, leaves, do)]
+    layouts = [make_layout(cu, r, ranks, balance) for r in range(ranks)]
+    exchanges = [OneGpu(r, max(layouts[0].rows_of_rank), T + TILE, 2 * Hkv * D) for r in range(ranks)]
+    for ex in exchanges:
+        ex.kv_ptrs, ex.dkv_ptrs = [e.kv.data_ptr() for e in exchanges], [e.dkv.data_ptr() for e in exchanges]
+        ex.kv_ptr_array = (_lib.c_void_p * ranks)(*ex.kv_ptrs)
+        ex.mirror_ptr_array = (_lib.c_void_p * 1)(ex.mirror.data_ptr())
+    rows = [torch.from_numpy(lay.local_index()).cuda() for lay in layouts]
+    local = [[t[i].clone().requires_grad_() for t in (q, k, v)] for i in rows]
+    for ex, (_, kl, vl) in zip(exchanges, local):
+        ex.publish(kl.detach(), vl.detach())
+    outs = [cp_attention(*local[r], layouts[r], build_cp_plan(layouts[r], torch.device("cuda", 0)), None, exchanges[r], Hq, Hkv)
+            for r in range(ranks)]
+    for _ in range(2):          # the first round fills every rank's staging rows, which the second one's owners then add
+        grads = [torch.autograd.grad(outs[r], local[r], do[rows[r]], retain_graph=True) for r in range(ranks)]
+    assert _lib.read_status() == 0
+    for r in range(ranks):
+        for name, got, full, tol in zip(("out", "dq", "dk", "dv"), (outs[r].detach(), *grads[r]), want, (2e-2, 3e-2, 3e-2, 3e-2)):
+            _close(got, full[rows[r]].float(), tol, f"rank {r} {name}")
