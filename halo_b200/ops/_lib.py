@@ -100,16 +100,21 @@ def stream_ptr(device: torch.device | None = None) -> c_void_p:
     return c_void_p(torch._C._cuda_getCurrentRawStream(index))
 
 
+# looked up once: the two conditions below run in front of every small kernel of a sampling step
+_forward_ad, _grad_enabled = torch.autograd.forward_ad, torch.is_grad_enabled
+_functorch_stack, _tracing = torch._C._functorch.peek_interpreter_stack, torch._C._is_tracing
+
+
 def untransformed() -> bool:
     """Nothing but reverse mode can be watching: no forward-mode differentiation, no functorch transform (vmap, grad, jvp), and no
     ``torch.jit.trace``, which records an autograd node as a call but cannot see what a kernel writes through a pointer."""
-    return (torch.autograd.forward_ad._current_level < 0 and torch._C._functorch.peek_interpreter_stack() is None
-            and not torch._C._is_tracing())
+    return _forward_ad._current_level < 0 and _functorch_stack() is None and not _tracing()
 
 
 def plain_inference() -> bool:
-    """True where an operation may call its kernels without its autograd node: the node would record and pass on nothing."""
-    return not torch.is_grad_enabled() and untransformed()
+    """True where an operation may call its kernels without its autograd node: gradients are off and the operation is
+    :func:`untransformed`, so the node would record and pass on nothing."""
+    return not _grad_enabled() and _forward_ad._current_level < 0 and _functorch_stack() is None and not _tracing()
 
 
 def check(rc: int, what: str) -> None:
