@@ -7,10 +7,12 @@
 // its columns (16 .. 256, padded to a power of two), and a cluster of up to 8 CTAs cuts the reduction, so that every SM
 // streams weights. Each CTA keeps a ring of 16 KB weight tiles in flight (two CTAs fit an SM, so one CTA's prologue and
 // epilogue run under the other's stream); the partial sums stay fp32, meet in distributed shared memory in a fixed order,
-// and every CTA of the cluster finishes its share of the tokens. No workspace, one launch.
+// and every CTA of the cluster finishes its share of the tokens. No workspace, one launch. The cuts and the choice of kernel follow
+// the number of tokens (few_rows_wins), so a token's result may differ in its last bit between calls of different sizes; calls
+// of one size repeat exactly.
 //
-// Measured (B200, weights cycled so that L2 does not hold them; the large-tile kernels / this one, us; floor = weight bytes
-// at the measured copy rate):
+// Measured (B200, weights cycled so that L2 does not hold them; the large-tile kernels as they were / this one, us; floor =
+// weight bytes at the measured copy rate; short reductions: see few_rows_wins):
 //   N x K             floor    M = 1          16             64             128            256
 //   4096 x 12288      15.4     69.7 / 22.8    69.9 / 23.8    69.9 / 24.8    71.0 / 28.2    71.4 / 39.7
 //   6144 x 4096        7.7     28.1 / 14.8    28.1 / 15.2    28.6 / 17.2    30.5 / 20.5    30.6 / 40.9
