@@ -542,8 +542,13 @@ int halo_gemm_bf16(const void* A, const void* B, void* C, void* aux, int M, int 
     const bool glu = epi == kEpiSwiglu;
     if (glu && N % 2) return -20;
     use_pair();                       // reads HALO_GEMM_PAIR: 2 sends every product to the pair kernel
-    if (g_use_pair != 2 && K > 0 && !a_mn_major && !b_mn_major && (epi == kEpiStoreBf16 || epi == kEpiStoreF32 || glu) &&
-        few_rows_wins(M, N, K, glu ? (N / 2 + 127) / 128 : (N + kBlockN - 1) / kBlockN, glu)) {
+    // The large tiles store 16 bytes at a time, the few-row kernel a pair of elements: outputs off the 16-byte boundary go to it as
+    // far as it reaches and are refused beyond.
+    const uintptr_t outs = reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(aux);
+    const bool aligned = (outs & 15u) == 0, pairs_aligned = (outs & (epi == kEpiStoreF32 ? 7u : 3u)) == 0;
+    const bool few_ok = K > 0 && !a_mn_major && !b_mn_major && (epi == kEpiStoreBf16 || epi == kEpiStoreF32 || glu);
+    if (!aligned && !(few_ok && M <= 256 && pairs_aligned)) return -23;
+    if (few_ok && (!aligned || (g_use_pair != 2 && few_rows_wins(M, N, K, glu ? (N / 2 + 127) / 128 : (N + kBlockN - 1) / kBlockN, glu)))) {
         FewParams f{};
         f.C = C; f.aux = aux; f.ldc = ldc; f.ld_aux = ld_aux; f.epi = epi; f.alpha = alpha;
         f.M = M; f.N = N; f.K = K; f.swiglu_f = glu ? N / 2 : 0; f.status = status;

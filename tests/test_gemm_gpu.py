@@ -236,3 +236,26 @@ def test_few_rows_from_several_threads():
     for _, out, _, _ in jobs:
         assert ((out - want).abs() <= 2.0 ** -8 * want.abs() + 0.05).all()
     assert _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(3, 40, 72), (64, 4096, 512), (100, 136, 64), (200, 24576, 128), (256, 520, 1000)])
+@pytest.mark.parametrize("f32", [False, True])
+def test_outputs_off_the_16_byte_boundary(M, N, K, f32):
+    """A few rows go to the kernel that stores pairs, whatever the reduction; what only the 16-byte kernels serve is refused."""
+    from halo_b200.ops import _lib
+    from halo_b200.ops.gemm import matmul
+
+    torch.manual_seed(N)
+    x, w = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+    buf = torch.full((M, N + 8), 7.0, device="cuda", dtype=torch.float32 if f32 else torch.bfloat16)
+    matmul(x, w, out=buf[:, 2:2 + N])
+    ref = x.double() @ w.double().t()
+    noise = K / 16 * 2.0 ** -23 * 5 * K ** 0.5 + 1e-6
+    assert ((buf[:, 2:2 + N] - ref).abs() <= (0.0 if f32 else 2.0 ** -8) * ref.abs() + noise).all()
+    assert (buf[:, :2] == 7.0).all() and (buf[:, 2 + N:] == 7.0).all() and _lib.read_status() == 0
+    for kwargs in ({"accumulate": True}, {"a_t": True}):
+        with pytest.raises((_lib.KernelError, ValueError)):         # a transposed operand of ragged M has no legal row stride
+            matmul(x.t().contiguous() if "a_t" in kwargs else x, w, out=buf[:, 2:2 + N], **kwargs)
+    tall = torch.zeros(300, N + 8, device="cuda", dtype=buf.dtype)
+    with pytest.raises(_lib.KernelError):
+        matmul(torch.zeros(300, K, device="cuda", dtype=torch.bfloat16), w, out=tall[:, 2:2 + N])
