@@ -73,10 +73,10 @@ def _scaled_bf16(x, g):
     return _round_and_scale(x, g)
 
 
-def _head_grad_buffer(weight, rows):
-    """fp32 sums of the head's gradient; the first row chunk stores into it, later ones accumulate."""
+def _head_grad_buffer(weight, rows, dtype=torch.float32):
+    """Sums of the head's gradient over the row chunks; the first stores into it, later ones accumulate."""
     new = torch.empty if rows else torch.zeros
-    return new(weight.shape, dtype=torch.float32, device=weight.device)
+    return new(weight.shape, dtype=dtype, device=weight.device)
 
 
 class _FusedLinearCE(torch.autograd.Function):
@@ -88,7 +88,8 @@ class _FusedLinearCE(torch.autograd.Function):
         need_dh = hidden.requires_grad
         need_dw = weight.requires_grad
         dh = torch.empty_like(hidden) if need_dh else None
-        dw32 = _head_grad_buffer(weight, T) if need_dw else None
+        one_chunk = T <= chunk_rows            # the product rounds its own fp32 sums: nothing to keep in fp32
+        dw = _head_grad_buffer(weight, T, torch.bfloat16 if one_chunk else torch.float32) if need_dw else None
         loss_sum = torch.zeros((), dtype=torch.float32, device=dev)
         Vp = (V + 7) // 8 * 8
         buf = torch.empty((min(chunk_rows, max(T, 1)), Vp), dtype=torch.bfloat16, device=dev)
@@ -102,9 +103,9 @@ class _FusedLinearCE(torch.autograd.Function):
             if need_dh:
                 matmul(logits, weight, b_t=False, out=dh[s:e])
             if need_dw:
-                matmul(logits, hc, a_t=True, b_t=False, out=dw32, accumulate=s > 0)
+                matmul(logits, hc, a_t=True, b_t=False, out=dw, accumulate=s > 0)
         # a pending loss holds the head's gradient in bf16, half of its sums: several may be pending at once
-        ctx.save_for_backward(dh, _round_and_scale(dw32) if need_dw else None)
+        ctx.save_for_backward(dh, dw if one_chunk or dw is None else _round_and_scale(dw))
         return loss_sum * grad_scale
 
     @staticmethod
