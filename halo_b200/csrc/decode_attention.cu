@@ -13,8 +13,8 @@
 // path: the group's G query heads against 16 keys are a 16 x 16 x head_dim product, done with mma.sync (a memory-bound
 // kernel needs 2 % of the tensor rate; tcgen05's 128-row tiles would be mostly padding).
 //
-// Precision: queries, keys and values are bf16 already, sums and softmax are fp32. The probabilities stay fp32 in effect:
-// each is split into two bf16 terms (p = hi + lo to 2^-17) that go through the same product. With G <= 8 the split is
+// Precision: queries, keys and values are bf16 already, sums and softmax are fp32. The probabilities that meet the values are
+// fp32 split into two bf16 terms (p = hi + lo, off by at most 2^-16 p) that go through the same product. With G <= 8 the split is
 // free: the product has 16 rows, the heads use rows 0-7 and the low terms ride in rows 8-15.
 //
 // Measured (B200, 64 sequences of 2,000-8,000 keys, 32 / 4 heads of 128: 655 MB of cache): 3,662 us before (one block of
